@@ -41,7 +41,7 @@ __global__ void geometry_kernel(Job job) {
   g.c0 = g.c1 = g.cstep = g.cf = 0.0f;
   g.offset = 0;
   g.valid = 0;
-  g.pad[0] = g.pad[1] = 0;
+  g.c0_lo = g.c1_lo = 0.0f;
   if (fabs(ndf) < 1.0e9) {  // false for NaN/Inf: flagged instead of undefined int()
     const int nd = __double2int_rz(__dadd_rn(ndf, 0.5));
     double frac = -__dmul_rn(__dsub_rn(ndf, (double)nd), job.Ts);
@@ -54,14 +54,16 @@ __global__ void geometry_kernel(Job job) {
     const double br = b - (double)intdelay;
     double c0 = br * job.lo_hz;
     if (job.fractional_lo) c0 += (job.lo_hz - trunc(job.lo_hz)) * (double)intdelay;
-    c0 -= floor(c0);
+    c0 -= rint(c0);
     const double c1 = a * job.lo_hz / (double)job.F;  // turns per sample
     // coarse step: the reference advances its step table by `stride` samples per
     // entry (fxkernel.cpp:112) while applying it every `substride` samples;
     // FXKERNEL mode keeps that, EXACT uses the true step.
     const double stepmul = (job.rotator == GXC_ROTATOR_FXKERNEL) ? (double)job.stride : (double)job.substride;
     g.c0 = (float)c0;
+    g.c0_lo = (float)(c0 - (double)g.c0);
     g.c1 = (float)c1;
+    g.c1_lo = (float)(c1 - (double)g.c1);
     g.cstep = (float)(c1 * stepmul);
     // fractional-sample correction exp(+2 pi i c bw/nchan frac) (fxkernel.cpp:171-175,600-630)
     g.cf = (float)(job.bw_hz / (double)job.nchan * frac);

@@ -499,16 +499,17 @@ __global__ void __launch_bounds__(NT, 1) fstage_tc_kernel(Params p) {
         if (!mbar_wait(smem_u32(&ab_full[s]), (c / NS) & 1, p.err)) break;
         if (c >= NS && !mbar_wait(smem_u32(&d_free[s]), ((c / NS) - 1) & 1, p.err)) break;
         tc_fence_after();
-        const uint32_t a1 = sbase + OFF_A1 + 2 * s * HB, b1 = sbase + OFF_B1 + 2 * s * KB;
+        const uint32_t a1 = desc_lo(sbase + OFF_A1 + 2 * s * HB), b1 = desc_lo(sbase + OFF_B1 + 2 * s * KB);
 #pragma unroll
         for (int part = 0; part < 2; part++)
 #pragma unroll
-          for (int pol = 0; pol < 2; pol++)
+          for (int pol = 0; pol < 2; pol++) {
+            const uint32_t d = tmem0 + 256u * s + 128 * part + ((uint32_t)(16 * pol) << 16);
+            const uint32_t a = a1 + part * HB / 16, b = b1 + pol * KB / 16;
+            mma_f16_lo<false>(d, a, b, IDESC_M64);
 #pragma unroll
-            for (int kk = 0; kk < 4; kk++)
-              mma_f16(tmem0 + 256u * s + 128 * part + ((uint32_t)(16 * pol) << 16),
-                      desc_sw128(a1 + part * HB + kk * 32), desc_sw128(b1 + pol * KB + kk * 32), IDESC_M64,
-                      kk > 0 ? 1u : 0u);
+            for (int kk = 1; kk < 4; kk++) mma_f16_lo<true>(d, a + 2 * kk, b + 2 * kk, IDESC_M64);
+          }
         mma_commit(smem_u32(&ab_free[s]));
         mma_commit(smem_u32(&d1_full[s]));
         c++;
@@ -527,11 +528,11 @@ __global__ void __launch_bounds__(NT, 1) fstage_tc_kernel(Params p) {
         const int s = c % NS;
         if (!mbar_wait(smem_u32(&a3_full[s]), (c / NS) & 1, p.err)) break;
         tc_fence_after();
-        const uint32_t d = tmem0 + 256u * s;
+        const uint32_t d = tmem0 + 256u * s, b3 = desc_lo(sbase + OFF_B3);
+        mma_f16_ts_lo<false>(d, d + 128, b3, IDESC);
 #pragma unroll
-        for (int kk = 0; kk < 16; kk++)
-          mma_f16_ts(d, d + 128 + 8 * kk, desc_sw128(sbase + OFF_B3 + (kk >> 2) * KB + (kk & 3) * 32), IDESC,
-                     kk > 0 ? 1u : 0u);
+        for (int kk = 1; kk < 16; kk++)
+          mma_f16_ts_lo<true>(d, d + 128 + 8 * kk, b3 + (kk >> 2) * KB / 16 + 2 * (kk & 3), IDESC);
         mma_commit(smem_u32(&d3_full[s]));
         c++;
       }

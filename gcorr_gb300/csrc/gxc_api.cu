@@ -27,6 +27,7 @@ struct gxc_handle {
   int chan_type = CHAN_F32;
   int xeng = GXC_XENGINE_CUDA_CORE;
   bool tc_fstage = false;  // tensor-core F-stage (fstage_tc.cu)
+  bool tc32_fstage = false;  // FP32-accurate F-stage with its first step on tensor cores (fstage_tc32.cu)
   void *d_tc_tables = nullptr;
   float out_scale = 1.f;   // applied to channelised values before the cast
   float vis_scale = 1.f;   // 1/out_scale^2, applied at finalisation
@@ -397,6 +398,8 @@ gxc_status gxc_create(const gxc_config *cfg, gxc_handle **out) {
   // 16-antenna, 512 Ms/s workload at FP16
   h->tc_fstage = cfg->fft_engine != GXC_FFT_CUDA_CORE && fstage_tc_supported(j, h->chan_type);
   if (e == cudaSuccess && h->tc_fstage) e = make_fstage_tc_tables(&h->d_tc_tables);
+  // otherwise the FP32-accurate F-stage: its first step on tensor cores where that is faster, else the register FFT
+  h->tc32_fstage = !h->tc_fstage && fstage_tc32_worth(j, h->T);
   if (h->chan_type == CHAN_F8 && cfg->fp8_scaling == GXC_FP8_SCALE_CHANNEL) {
     // calibration block: up to 64 FFTs, at most 256 MB of FP32 channelised data (at least 4 FFTs)
     const size_t per_fft32 = (size_t)cfg->nchan * 2 * nant * sizeof(float2);
@@ -762,6 +765,9 @@ extern "C++" gxc_status gxc::process_chained(gxc_handle *h, void *stream, cudaEv
       GXC_CUDA(h, launch_fstage_tc(h->job, h->d_tc_tables, t0, nt, h->T, h->d_chan, h->chan_type, osc, s,
                                    h->d_cscale),
                "tensor-core F-stage kernel");
+    else if (h->tc32_fstage)
+      GXC_CUDA(h, launch_fstage_tc32(h->job, t0, nt, h->T, h->d_chan, h->chan_type, osc, s, h->d_cscale),
+               "tensor-core assisted F-stage kernel");
     else
       GXC_CUDA(h, launch_fstage(h->job, h->d_tw, t0, nt, h->T, h->d_chan, h->chan_type, osc, s, h->d_cscale),
                "F-stage kernel");
@@ -825,6 +831,8 @@ gxc_status gxc_probe_unpack(gxc_handle *h, float *decoded) {
     // the probe runs the handle's own F-stage kernel family
     e = h->tc_fstage ? launch_fstage_tc(h->job, h->d_tc_tables, t0, nt, h->T, chan, h->chan_type, h->out_scale,
                                         nullptr, nullptr, probe)
+        : h->tc32_fstage ? launch_fstage_tc32(h->job, t0, nt, h->T, chan, h->chan_type, h->out_scale, nullptr, nullptr,
+                                              probe)
                      : launch_fstage_probe(h->job, h->d_tw, t0, nt, h->T, chan, h->chan_type, h->out_scale, probe,
                                            nullptr);
   }
@@ -851,6 +859,11 @@ gxc_status gxc_sync(gxc_handle *h) {
     int flag = 0;
     GXC_CUDA(h, fstage_tc_take_error(&flag), "reading the F-stage status");
     if (flag) return fail(h, GXC_ERR_TIMEOUT, "tensor-core F-stage: a bounded device wait expired");
+  }
+  if (h->tc32_fstage) {
+    int flag = 0;
+    GXC_CUDA(h, fstage_tc32_take_error(&flag), "reading the F-stage status");
+    if (flag) return fail(h, GXC_ERR_TIMEOUT, "tensor-core assisted F-stage: a bounded device wait expired");
   }
   return GXC_OK;
 }

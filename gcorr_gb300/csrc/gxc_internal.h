@@ -19,13 +19,14 @@ constexpr int CW = 16;
 // constants of the F-stage are evaluated there in FP64, once per (antenna, FFT),
 // reduced mod 1 turn and rounded to FP32 (fxkernel.cpp:503-535, :600-630).
 struct Geom {
-  float c0;      // fringe phase at the first sample, turns, in [0, 1)
+  float c0;      // fringe phase at the first sample, turns, in [-1/2, 1/2]
   float c1;      // fringe phase slope, turns per sample
   float cstep;   // phase advance of one coarse rotator-table entry, turns
   float cf;      // fractional-sample correction, turns per channel
   int offset;    // first sample of the FFT window in the antenna stream
   int valid;     // 0 = flagged (window outside the buffer)
-  int pad[2];
+  float c0_lo;   // the rest of the fringe phase: c0 + c0_lo holds it to about 48 bits
+  float c1_lo;   // the rest of the phase slope
 };
 static_assert(sizeof(Geom) == 32, "Geom layout");
 
@@ -80,6 +81,14 @@ cudaError_t launch_fstage_tc(const Job &job, const void *tables, int t0, int nt,
                              float out_scale, cudaStream_t s, const float *cscale = nullptr,
                              float2 *probe = nullptr);
 cudaError_t fstage_tc_take_error(int *flag);
+
+// fstage_tc32.cu: the F-stage in FP32 accuracy with its first step on tensor cores (2048- to 8192-point windows, 2-bit
+// real), every channelised type.  T: the handle's FFT block.  probe as for launch_fstage_tc.
+int fstage_tc32_supported(const Job &job, int T);
+int fstage_tc32_worth(const Job &job, int T);  // supported, and faster than the register FFT at this size
+cudaError_t launch_fstage_tc32(const Job &job, int t0, int nt, int T, void *chan, int chan_type, float out_scale,
+                               cudaStream_t s, const float *cscale = nullptr, float2 *probe = nullptr);
+cudaError_t fstage_tc32_take_error(int *flag);
 
 // xstage_fp32.cu: accumulates visibilities of FFTs [0, nt) of the block into
 // the compensated (sum, comp) accumulators in the output layout.
