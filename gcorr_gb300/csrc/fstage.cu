@@ -18,17 +18,19 @@
 namespace gxc {
 
 // ----------------------------------------------------------------- geometry
-// One thread per (antenna, FFT).  FP64 with explicit round-to-nearest
+// One thread per (antenna, FFT), antenna a0 + blockIdx.y.  FP64 with explicit round-to-nearest
 // operations so the integer/fractional split matches the CPU reference bit
 // for bit (no FMA contraction): fxkernel.cpp:432-439 and :289-309.
-__global__ void geometry_kernel(Job job) {
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long total = (long long)job.nant * job.nfft;
-  if (idx >= total) return;
-  const int ant = (int)(idx / job.nfft);
-  const int i = (int)(idx % job.nfft);
-  const double *p = job.poly + 3 * ant;
-  const double fso = job.fso[ant];
+// The per-call parameters (input pointers, delay model) arrive as kernel parameters; the first block of an antenna
+// writes its input pointer where the F-stage reads it.  Validity also goes out as one bit per FFT (vbits [nant][nw]).
+// Bound by the FP64 pipe (two operations per clock and SM).
+__global__ void geometry_kernel(Job job, const __grid_constant__ GeomParams u, int nw, uint32_t *__restrict__ vbits) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int al = blockIdx.y, ant = u.a0 + al;
+  if (i == 0) job.inputs[ant] = u.ptrs[al];
+  const bool in_range = i < job.nfft;
+  const double *p = u.poly + 3 * al;
+  const double fso = u.fso[al];
   const double fi = (double)i, fh = fi + 0.5, f1 = fi + 1.0;
   const double d0 = __dadd_rn(__dadd_rn(__dmul_rn(__dmul_rn(p[0], fi), fi), __dmul_rn(p[1], fi)), p[2]);
   const double d1 = __dadd_rn(__dadd_rn(__dmul_rn(__dmul_rn(p[0], fh), fh), __dmul_rn(p[1], fh)), p[2]);
@@ -55,7 +57,7 @@ __global__ void geometry_kernel(Job job) {
     double c0 = br * job.lo_hz;
     if (job.fractional_lo) c0 += (job.lo_hz - trunc(job.lo_hz)) * (double)intdelay;
     c0 -= rint(c0);
-    const double c1 = a * job.lo_hz / (double)job.F;  // turns per sample
+    const double c1 = a * job.lo_hz * job.inv_F;  // turns per sample (F is a power of two)
     // coarse step: the reference advances its step table by `stride` samples per
     // entry (fxkernel.cpp:112) while applying it every `substride` samples;
     // FXKERNEL mode keeps that, EXACT uses the true step.
@@ -66,70 +68,48 @@ __global__ void geometry_kernel(Job job) {
     g.c1_lo = (float)(c1 - (double)g.c1);
     g.cstep = (float)(c1 * stepmul);
     // fractional-sample correction exp(+2 pi i c bw/nchan frac) (fxkernel.cpp:171-175,600-630)
-    g.cf = (float)(job.bw_hz / (double)job.nchan * frac);
+    g.cf = (float)(job.bw_chan * frac);
     if (off >= 0 && off <= job.maxoffset) {
       g.offset = (int)off;
       g.valid = 1;
-      const uint8_t *fv = job.fvalid ? job.fvalid[ant] : nullptr;
-      if (fv) {
+      const uint8_t *fv = u.fvalid[al];
+      if (fv && in_range) {
         const long long f1 = (off + job.F - 1) / job.samples_per_frame;
         for (long long f = off / job.samples_per_frame; f <= f1; f++)
           if (!fv[f]) g.valid = 0;
       }
     }
   }
-  job.geom[idx] = g;
+  if (in_range) job.geom[(size_t)ant * job.nfft + i] = g;
+  const uint32_t bits = __ballot_sync(0xffffffffu, in_range && g.valid);
+  if ((threadIdx.x & 31) == 0 && (i >> 5) < nw) vbits[(size_t)ant * nw + (i >> 5)] = bits;
 }
 
-cudaError_t launch_geometry(const Job &job, cudaStream_t s) {
-  const long long total = (long long)job.nant * job.nfft;
-  const int threads = 256;
-  const long long blocks = (total + threads - 1) / threads;
-  geometry_kernel<<<(unsigned)blocks, threads, 0, s>>>(job);
+cudaError_t launch_geometry(const Job &job, const GeomParams &u, int n, uint32_t *vbits, cudaStream_t s) {
+  const int threads = 256, nw = (job.nfft + 31) / 32;
+  dim3 grid((unsigned)((job.nfft + threads - 1) / threads), (unsigned)n);
+  geometry_kernel<<<grid, threads, 0, s>>>(job, u, nw, vbits);
   return cudaGetLastError();
 }
 
 // ------------------------------------------------------------------- counts
-// counts[bl] = number of FFTs where both antennas are valid (fxkernel.cpp:352),
-// plus the antValid flags exported as uint8 [nant][nfft].
-__global__ void counts_kernel(const Geom *__restrict__ geom, int nant, int nfft, int autos, int32_t *counts,
-                              uint8_t *valid_flags) {
+// counts[bl] = number of FFTs where both antennas are valid (fxkernel.cpp:352), from the validity bits.  One CTA per
+// baseline: 5 us for 16 antennas and 62500 FFTs (275 us when it read the geometry records and one CTA exported every
+// flag).
+__global__ void counts_kernel(const uint32_t *__restrict__ vbits, int nant, int nw, int32_t *counts) {
   const int bl = blockIdx.x;
-  const int ncross = nant * (nant - 1) / 2;
   int j, k;
-  if (bl >= ncross) {
-    j = k = bl - ncross;
-  } else {  // invert the fxkernel baseline order
-    j = 0;
-    int rem = bl;
-    while (rem >= nant - 1 - j) { rem -= nant - 1 - j; j++; }
-    k = j + 1 + rem;
-  }
+  baseline_antennas(bl, nant, &j, &k);
   int c = 0;
-  for (int t = threadIdx.x; t < nfft; t += blockDim.x) {
-    const int vj = geom[(size_t)j * nfft + t].valid;
-    const int vk = geom[(size_t)k * nfft + t].valid;
-    c += (vj && vk) ? 1 : 0;
-    if (valid_flags && bl == 0) {
-      // block 0 also exports every antenna's flags
-      for (int a = 0; a < nant; a++) valid_flags[(size_t)a * nfft + t] = (uint8_t)geom[(size_t)a * nfft + t].valid;
-    }
-  }
-  __shared__ int red[32];
-  for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = c;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    int v = (threadIdx.x < (int)(blockDim.x >> 5)) ? red[threadIdx.x] : 0;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (threadIdx.x == 0) counts[bl] = v;
-  }
+  for (int w = threadIdx.x; w < nw; w += blockDim.x)
+    c += __popc(vbits[(size_t)j * nw + w] & vbits[(size_t)k * nw + w]);
+  c = block_sum256(c);
+  if (threadIdx.x == 0) counts[bl] = c;
 }
 
-cudaError_t launch_counts(const Job &job, int autos, int32_t *counts, uint8_t *valid_flags, cudaStream_t s) {
-  const int nbl = job.nant * (job.nant - 1) / 2 + (autos ? job.nant : 0);
+cudaError_t launch_counts(const uint32_t *vbits, int nant, int nfft, int nbl, int32_t *counts, cudaStream_t s) {
   if (nbl == 0) return cudaSuccess;
-  counts_kernel<<<nbl, 256, 0, s>>>(job.geom, job.nant, job.nfft, autos, counts, valid_flags);
+  counts_kernel<<<nbl, 256, 0, s>>>(vbits, nant, (nfft + 31) / 32, counts);
   return cudaGetLastError();
 }
 

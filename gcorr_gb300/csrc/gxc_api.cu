@@ -50,20 +50,18 @@ struct gxc_handle {
   std::vector<cudaEvent_t> in_chunk_ev;
   std::vector<long long> in_chunk_end;
   const uint8_t **d_inptrs = nullptr;  // device array of per-antenna device pointers
-  double *d_poly = nullptr, *d_fso = nullptr;
-  // frame validity (gxc_set_frame_validity): user device pointers, uploaded per process()
+  // frame validity (gxc_set_frame_validity): user device pointers, passed on per process()
   std::vector<const uint8_t *> user_fvalid;
-  const uint8_t **d_fvalid = nullptr;
   std::vector<double> poly, fso;
 
   // state
   Geom *d_geom = nullptr;
   int32_t *d_counts = nullptr;
-  uint8_t *d_valid = nullptr;
+  uint32_t *d_vbits = nullptr;  // validity, one bit per FFT: [nant][(nfft + 31) / 32]
   float2 *d_tw = nullptr;
   int2 *d_pairs = nullptr;  // tile pairs of the CUDA-core X-stage
   void *d_chan = nullptr;
-  float2 *d_vsum = nullptr, *d_vcomp = nullptr, *d_vis = nullptr;
+  float2 *d_acc = nullptr, *d_vis = nullptr;  // accumulators: two planes of (sum, compensation)
   cudaStream_t last_stream = nullptr;
   cudaEvent_t ev_done = nullptr;
   bool processed = false;
@@ -245,12 +243,9 @@ const float *gxc_device_visibilities(const gxc_handle *h) { return h ? (const fl
 static void release(gxc_handle *h) {
   cudaFree(h->d_inbuf);
   cudaFree((void *)h->d_inptrs);
-  cudaFree(h->d_poly);
-  cudaFree(h->d_fso);
-  cudaFree((void *)h->d_fvalid);
   cudaFree(h->d_geom);
   cudaFree(h->d_counts);
-  cudaFree(h->d_valid);
+  cudaFree(h->d_vbits);
   cudaFree(h->d_tw);
   cudaFree(h->d_tc_tables);
   cudaFree(h->d_cal);
@@ -258,8 +253,7 @@ static void release(gxc_handle *h) {
   cudaFree(h->d_cvscale);
   cudaFree(h->d_pairs);
   cudaFree(h->d_chan);
-  cudaFree(h->d_vsum);
-  cudaFree(h->d_vcomp);
+  cudaFree(h->d_acc);
   cudaFree(h->d_vis);
   if (h->ev_done) cudaEventDestroy(h->ev_done);
   if (h->ev_fork) cudaEventDestroy(h->ev_fork);
@@ -370,7 +364,8 @@ gxc_status gxc_create(const gxc_config *cfg, gxc_handle **out) {
   j.bw_hz = cfg->bw_hz;
   j.Ts = cfg->is_complex ? 1.0 / cfg->bw_hz : 1.0 / (2.0 * cfg->bw_hz);
   j.maxoffset = (long long)(cfg->nfft - 1) * h->F;
-  j.fvalid = nullptr;
+  j.inv_F = 1.0 / (double)h->F;
+  j.bw_chan = cfg->bw_hz / (double)cfg->nchan;
   j.samples_per_frame = 0;
 
   cudaError_t e = cudaSuccess;
@@ -378,18 +373,14 @@ gxc_status gxc_create(const gxc_config *cfg, gxc_handle **out) {
     if (e == cudaSuccess) e = cudaMalloc(p, n);
   };
   A((void **)&h->d_inptrs, sizeof(uint8_t *) * nant);
-  A((void **)&h->d_poly, sizeof(double) * 3 * nant);
-  A((void **)&h->d_fso, sizeof(double) * nant);
-  A((void **)&h->d_fvalid, sizeof(uint8_t *) * nant);
   A((void **)&h->d_geom, sizeof(Geom) * (size_t)nant * cfg->nfft);
   A((void **)&h->d_counts, sizeof(int32_t) * (h->nbl > 0 ? h->nbl : 1));
-  A((void **)&h->d_valid, (size_t)nant * cfg->nfft);
+  A((void **)&h->d_vbits, sizeof(uint32_t) * (size_t)nant * ((cfg->nfft + 31) / 32));
   A(&h->d_chan, per_fft * (size_t)T);
   const size_t nvis = (size_t)(h->nbl > 0 ? h->nbl : 1) * 4 * cfg->nchan;
   // two accumulator planes: the tensor X-stage may split a block's FFTs across two CTAs per
   // channel group (launch_xstage_tensor); finalisation sums the planes
-  A((void **)&h->d_vsum, sizeof(float2) * nvis * 2);
-  A((void **)&h->d_vcomp, sizeof(float2) * nvis * 2);
+  A((void **)&h->d_acc, sizeof(float2) * nvis * 4);
   A((void **)&h->d_vis, sizeof(float2) * nvis);
   if (e == cudaSuccess) e = make_twiddles(h->F, &h->d_tw);
   if (e == cudaSuccess) e = make_tile_pairs(nant, &h->d_pairs);
@@ -421,8 +412,6 @@ gxc_status gxc_create(const gxc_config *cfg, gxc_handle **out) {
     return e == cudaErrorMemoryAllocation ? GXC_ERR_OUT_OF_MEMORY : GXC_ERR_CUDA;
   }
   j.inputs = h->d_inptrs;
-  j.poly = h->d_poly;
-  j.fso = h->d_fso;
   j.geom = h->d_geom;
   h->poly.assign(3 * (size_t)nant, 0.0);
   h->fso.assign((size_t)nant, 0.0);
@@ -502,7 +491,6 @@ gxc_status gxc_set_frame_validity(gxc_handle *h, const uint8_t *const *valid, si
   if (!h) return GXC_ERR_INVALID_ARGUMENT;
   if (!valid) {
     h->user_fvalid.clear();
-    h->job.fvalid = nullptr;
     h->job.samples_per_frame = 0;
     return GXC_OK;
   }
@@ -523,7 +511,6 @@ gxc_status gxc_set_frame_validity(gxc_handle *h, const uint8_t *const *valid, si
     }
   }
   h->user_fvalid.assign(valid, valid + h->cfg.nant);
-  h->job.fvalid = h->d_fvalid;
   h->job.samples_per_frame = samples_per_frame;
   return GXC_OK;
 }
@@ -584,23 +571,50 @@ static cudaError_t launch_chan_scales(const float2 *cal, int nstream, int nchan,
   return cudaGetLastError();
 }
 
+}  // extern "C"
+
 // finalisation: vis = (sum + comp) * scale / count (fxkernel.cpp:358-367)
-// Sums the two accumulator planes (i and i + n) with a compensated add; a plane no launch wrote
-// is zero and leaves the result bit-identical to the first plane's.
-__global__ void finalize_kernel(const float2 *__restrict__ vsum, const float2 *__restrict__ vcomp,
-                                const int32_t *__restrict__ counts, int nchan, size_t n, float scale,
-                                const float *__restrict__ chan_vscale,
-                                float2 *__restrict__ vis) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+// plane > 0: adds the second accumulator plane (plane elements further) with a compensated add.
+// COUNT: the block also counts its baseline's FFTs, from the validity bits (short sub-integrations: one launch less;
+// otherwise counts_kernel has run).  A block's 256 values belong to one baseline (nchan >= 128).
+template <bool COUNT>
+__global__ void __launch_bounds__(256) finalize_kernel(const float2 *__restrict__ vsum, const float2 *__restrict__ vcomp,
+                                                       size_t plane, int32_t *__restrict__ counts,
+                                                       const uint32_t *__restrict__ vbits, int nant, int nw, int nchan,
+                                                       size_t n, float scale, const float *__restrict__ chan_vscale,
+                                                       float2 *__restrict__ vis) {
+  const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+  const int bl = (int)(((size_t)blockIdx.x * 256) / ((size_t)4 * nchan));
+  int cnt;
+  if constexpr (COUNT) {
+    __shared__ int total;
+    int j, k;
+    baseline_antennas(bl, nant, &j, &k);
+    int c = (int)threadIdx.x < nw
+                ? __popc(vbits[(size_t)j * nw + threadIdx.x] & vbits[(size_t)k * nw + threadIdx.x])
+                : 0;
+    c = block_sum256(c);
+    if (threadIdx.x == 0) {
+      total = c;
+      counts[bl] = c;
+    }
+    __syncthreads();
+    cnt = total;
+  } else {
+    cnt = counts[bl];
+  }
   if (i >= n) return;
-  const int bl = (int)(i / ((size_t)4 * nchan));
-  const int cnt = counts[bl];
-  const float2 s0 = vsum[i], c0 = vcomp[i], s1 = vsum[i + n], c1 = vcomp[i + n];
+  const float2 s0 = vsum[i], c0 = vcomp[i];
   float sx = s0.x, ex = c0.x, sy = s0.y, ey = c0.y;
-  two_sum_add(sx, ex, s1.x);
-  two_sum_add(sy, ey, s1.y);
+  if (plane) {
+    const float2 s1 = vsum[i + plane], c1 = vcomp[i + plane];
+    two_sum_add(sx, ex, s1.x);
+    two_sum_add(sy, ey, s1.y);
+    ex += c1.x;
+    ey += c1.y;
+  }
   const float sc = chan_vscale ? chan_vscale[i % nchan] : scale;
-  float re = (sx + (ex + c1.x)) * sc, im = (sy + (ey + c1.y)) * sc;
+  float re = (sx + ex) * sc, im = (sy + ey) * sc;
   if (cnt > 0) {
     re /= (float)cnt;
     im /= (float)cnt;
@@ -608,26 +622,7 @@ __global__ void finalize_kernel(const float2 *__restrict__ vsum, const float2 *_
   vis[i] = make_float2(re, im);
 }
 
-// Per-call parameters of up to kAnt antennas (about 10 KB: kernel parameters of up to
-// 32 KB are allowed on this architecture).
-struct UploadChunk {
-  static constexpr int kAnt = 256;
-  int a0, n;
-  const uint8_t *ptrs[kAnt];
-  const uint8_t *fvalid[kAnt];
-  double poly[3 * kAnt];
-  double fso[kAnt];
-};
-
-__global__ void upload_kernel(const __grid_constant__ UploadChunk u, const uint8_t **d_ptrs, double *d_poly,
-                              double *d_fso, const uint8_t **d_fvalid) {
-  for (int i = threadIdx.x; i < u.n; i += blockDim.x) {
-    d_ptrs[u.a0 + i] = u.ptrs[i];
-    d_fvalid[u.a0 + i] = u.fvalid[i];
-    d_fso[u.a0 + i] = u.fso[i];
-    for (int j = 0; j < 3; j++) d_poly[3 * (u.a0 + i) + j] = u.poly[3 * i + j];
-  }
-}
+extern "C" {
 
 __global__ void add_kernel(float *__restrict__ dst, const float *__restrict__ src, size_t n) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -651,9 +646,6 @@ extern "C++" gxc_status gxc::process_chained(gxc_handle *h, void *stream, cudaEv
   const int nant = c.nant;
   int launches = 0;
 
-  // input pointers and the delay model travel as kernel parameters of a one-block upload
-  // kernel (no host->device memcpy on the stream: small copies would queue on the copy
-  // engine behind bulk input copies of other streams, and need no host wait here)
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   GXC_CUDA(h, cudaStreamIsCapturing(s, &cap), "querying stream capture");
   const bool capturing = cap != cudaStreamCaptureStatusNone;
@@ -661,21 +653,6 @@ extern "C++" gxc_status gxc::process_chained(gxc_handle *h, void *stream, cudaEv
   // so sync() and the getters wait for the latest graph launch; stage timing is off there
   const unsigned rec_flags = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
   const bool timing = h->stage_timing && !capturing;
-  for (int a0 = 0; a0 < nant; a0 += UploadChunk::kAnt) {
-    UploadChunk u;
-    u.a0 = a0;
-    u.n = nant - a0 < UploadChunk::kAnt ? nant - a0 : UploadChunk::kAnt;
-    for (int i = 0; i < u.n; i++) {
-      const int a = a0 + i;
-      u.ptrs[i] = h->input_on_host ? h->d_inbuf + (size_t)a * h->bytes_per_ant : h->user_ptrs[a];
-      for (int j = 0; j < 3; j++) u.poly[3 * i + j] = h->poly[3 * (size_t)a + j];
-      u.fso[i] = h->fso[a];
-      u.fvalid[i] = h->user_fvalid.empty() ? nullptr : h->user_fvalid[a];
-    }
-    upload_kernel<<<1, 128, 0, s>>>(u, h->d_inptrs, h->d_poly, h->d_fso, h->d_fvalid);
-    GXC_CUDA(h, cudaGetLastError(), "upload kernel");
-    launches++;
-  }
   if (h->input_on_host) {
     // host inputs: copied on the handle's copy stream (forked from s) in time-ordered chunks, so
     // the F-stage blocks below start while later samples still load
@@ -711,15 +688,33 @@ extern "C++" gxc_status gxc::process_chained(gxc_handle *h, void *stream, cudaEv
   }
   if (timing) GXC_CUDA(h, cudaEventRecord(h->ev_begin, s), "timing event");
 
-  GXC_CUDA(h, launch_geometry(h->job, s), "geometry kernel");
-  launches++;
-  if (h->nbl > 0) {
-    GXC_CUDA(h, launch_counts(h->job, c.autos, h->d_counts, h->d_valid, s), "counts kernel");
+  // input pointers and the delay model travel as kernel parameters of the geometry kernel (no
+  // host->device memcpy on the stream: small copies would queue on the copy engine behind bulk
+  // input copies of other streams, and need no host wait here)
+  for (int a0 = 0; a0 < nant; a0 += GeomParams::kAnt) {
+    GeomParams u;
+    u.a0 = a0;
+    const int n = nant - a0 < GeomParams::kAnt ? nant - a0 : GeomParams::kAnt;
+    for (int i = 0; i < n; i++) {
+      const int a = a0 + i;
+      u.ptrs[i] = h->input_on_host ? h->d_inbuf + (size_t)a * h->bytes_per_ant : h->user_ptrs[a];
+      for (int j = 0; j < 3; j++) u.poly[3 * i + j] = h->poly[3 * (size_t)a + j];
+      u.fso[i] = h->fso[a];
+      u.fvalid[i] = h->user_fvalid.empty() ? nullptr : h->user_fvalid[a];
+    }
+    GXC_CUDA(h, launch_geometry(h->job, u, n, h->d_vbits, s), "geometry kernel");
+    launches++;
+  }
+  // up to 256 words of validity bits (8192 FFTs) finalisation counts the baselines' FFTs itself
+  const int nw = (c.nfft + 31) / 32;
+  const bool count_late = nw <= 256;
+  if (h->nbl > 0 && !count_late) {
+    GXC_CUDA(h, launch_counts(h->d_vbits, nant, c.nfft, h->nbl, h->d_counts, s), "counts kernel");
     launches++;
   }
   const size_t nvis = (size_t)h->nbl * 4 * c.nchan;
-  GXC_CUDA(h, cudaMemsetAsync(h->d_vsum, 0, sizeof(float2) * nvis * 2, s), "clearing accumulators");
-  GXC_CUDA(h, cudaMemsetAsync(h->d_vcomp, 0, sizeof(float2) * nvis * 2, s), "clearing accumulators");
+  float2 *const vsum = h->d_acc, *const vcomp = h->d_acc + nvis;
+  const size_t plane = 2 * nvis;  // the second plane's sum and compensation follow the first's
 
   // blocks: T FFTs each; with host inputs T0, 2 T0, 4 T0, ... up to T
   h->blk.clear();
@@ -734,6 +729,15 @@ extern "C++" gxc_status gxc::process_chained(gxc_handle *h, void *stream, cudaEv
     for (cudaEvent_t e : h->ev_stage) cudaEventDestroy(e);
     h->ev_stage.assign((size_t)3 * h->nblocks, nullptr);
     for (auto &e : h->ev_stage) GXC_CUDA(h, cudaEventCreate(&e), "timing event");
+  }
+  // the first block stores its sums, so the first plane needs no clearing; the second one does where it is used
+  const int kparts = c.x_split == GXC_XSPLIT_OFF ? 1 : c.x_split == GXC_XSPLIT_ON ? 3 : 2;
+  bool two_planes = false;
+  if (h->xeng == GXC_XENGINE_TENSOR && h->nbl > 0) {
+    for (const auto &blk : h->blk)
+      two_planes = two_planes || xstage_tensor_uses_plane(nant, c.nchan, h->chan_type, blk.second, kparts);
+    if (two_planes)
+      GXC_CUDA(h, cudaMemsetAsync(vsum + plane, 0, sizeof(float2) * plane, s), "clearing accumulators");
   }
   int waited = -1;  // input chunks already waited for
   for (int b = 0; b < h->nblocks; b++) {
@@ -779,14 +783,13 @@ extern "C++" gxc_status gxc::process_chained(gxc_handle *h, void *stream, cudaEv
         // at most F * 128*sqrt(2) (8-bit complex; 2-bit real is below that), which after the scale
         // is <= 2^ceil(log2F/2) * 182 <= 46592 < 65504, the FP16 maximum, for every F <= 32768.
         GXC_CUDA(h,
-                 launch_xstage_tensor(h->d_chan, h->chan_type, nant, c.nchan, h->T, nt, c.autos, h->d_vsum,
-                                      h->d_vcomp, s, h->log2F / 2,
-                                      c.x_split == GXC_XSPLIT_OFF ? 1 : c.x_split == GXC_XSPLIT_ON ? 3 : 2, nvis),
+                 launch_xstage_tensor(h->d_chan, h->chan_type, nant, c.nchan, h->T, nt, c.autos, vsum, vcomp, s,
+                                      h->log2F / 2, kparts, plane, b == 0),
                  "tensor-core X-stage kernel");
       } else {
         GXC_CUDA(h,
                  launch_xstage_cuda_core(h->d_chan, h->chan_type, nant, c.nchan, h->T, nt, c.autos, h->d_pairs,
-                                         h->d_vsum, h->d_vcomp, s),
+                                         vsum, vcomp, s, b == 0),
                  "X-stage kernel");
       }
       launches++;
@@ -796,9 +799,9 @@ extern "C++" gxc_status gxc::process_chained(gxc_handle *h, void *stream, cudaEv
   // join the input copies (the last blocks may not need the last chunk)
   if (nchunk > 0) GXC_CUDA(h, cudaStreamWaitEvent(s, chunk_ev[nchunk - 1], 0), "joining the input copies");
   if (nvis > 0) {
-    const int th = 256;
-    finalize_kernel<<<(unsigned)((nvis + th - 1) / th), th, 0, s>>>(h->d_vsum, h->d_vcomp, h->d_counts, c.nchan,
-                                                                     nvis, h->vis_scale, h->d_cvscale, h->d_vis);
+    auto fin = count_late ? finalize_kernel<true> : finalize_kernel<false>;
+    fin<<<(unsigned)((nvis + 255) / 256), 256, 0, s>>>(vsum, vcomp, two_planes ? plane : 0, h->d_counts, h->d_vbits, nant,
+                                                       nw, c.nchan, nvis, h->vis_scale, h->d_cvscale, h->d_vis);
     GXC_CUDA(h, cudaGetLastError(), "finalize kernel");
     launches++;
   }
@@ -926,8 +929,12 @@ gxc_status gxc_get_valid_flags(gxc_handle *h, uint8_t *flags) {
   if (h->nbl == 0) return fail(h, GXC_ERR_STATE, "no baselines: flags are not exported");
   gxc_status st = gxc_sync(h);
   if (st != GXC_OK) return st;
-  GXC_CUDA(h, cudaMemcpy(flags, h->d_valid, (size_t)h->cfg.nant * h->cfg.nfft, cudaMemcpyDeviceToHost),
+  const int nant = h->cfg.nant, nfft = h->cfg.nfft, nw = (nfft + 31) / 32;
+  std::vector<uint32_t> bits((size_t)nant * nw);
+  GXC_CUDA(h, cudaMemcpy(bits.data(), h->d_vbits, bits.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost),
            "copying flags");
+  for (int a = 0; a < nant; a++)
+    for (int t = 0; t < nfft; t++) flags[(size_t)a * nfft + t] = (bits[(size_t)a * nw + (t >> 5)] >> (t & 31)) & 1u;
   return GXC_OK;
 }
 

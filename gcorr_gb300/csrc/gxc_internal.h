@@ -32,9 +32,7 @@ static_assert(sizeof(Geom) == 32, "Geom layout");
 
 // Launch-time description of one sub-integration for the device kernels.
 struct Job {
-  const uint8_t *const *inputs;  // device array of nant device pointers
-  const double *poly;            // [nant][3]
-  const double *fso;             // [nant]
+  const uint8_t **inputs;        // device array of nant device pointers
   Geom *geom;                    // [nant][nfft]
   int nant, nchan, nfft, F, log2F;
   int is_complex;                // 0: 2-bit real, 1: 8-bit complex
@@ -43,11 +41,9 @@ struct Job {
   int fsub, fstride;             // frac-delay table split: nchan = fstride * fsub
   int fractional_lo;             // fxkernel.cpp:67-71
   double lo_hz, bw_hz, Ts;
+  double inv_F, bw_chan;         // 1 / F and bw_hz / nchan (exact: powers of two)
   long long maxoffset;           // (nfft-1)*F
-  // optional per-antenna frame validity (e.g. from a VDIF depacketiser): device array of nant
-  // pointers to uint8 [nframes] (a null entry = all valid); an FFT whose window touches an
-  // invalid frame is flagged.  fvalid == nullptr: no frame flags.
-  const uint8_t *const *fvalid;
+  // frame length of the optional per-antenna frame validity (GeomParams::fvalid)
   long long samples_per_frame;
 };
 
@@ -59,9 +55,22 @@ inline int chan_type_of(int precision) {
   return precision == GXC_PRECISION_FP32 ? CHAN_F32 : precision == GXC_PRECISION_FP16 ? CHAN_F16 : CHAN_F8;
 }
 
-// fstage.cu
-cudaError_t launch_geometry(const Job &job, cudaStream_t s);
-cudaError_t launch_counts(const Job &job, int autos, int32_t *counts, uint8_t *valid_flags, cudaStream_t s);
+// Per-call parameters of up to kAnt antennas, passed to the geometry kernel by value (about 12 KB: kernel parameters
+// of up to 32 KB are allowed on this architecture).  fvalid: optional per-antenna frame validity (e.g. from a VDIF
+// depacketiser), uint8 [nframes] in device memory, or null = all valid; an FFT whose window touches an invalid frame
+// is flagged.
+struct GeomParams {
+  static constexpr int kAnt = 256;
+  int a0;
+  const uint8_t *ptrs[kAnt];
+  const uint8_t *fvalid[kAnt];
+  double poly[3 * kAnt];
+  double fso[kAnt];
+};
+
+// fstage.cu: geometry records, input pointers and validity bits (vbits [nant][(nfft + 31) / 32]) of n antennas
+cudaError_t launch_geometry(const Job &job, const GeomParams &u, int n, uint32_t *vbits, cudaStream_t s);
+cudaError_t launch_counts(const uint32_t *vbits, int nant, int nfft, int nbl, int32_t *counts, cudaStream_t s);
 cudaError_t make_twiddles(int F, float2 **out);
 // cscale (FP8 output only): per-channel output scale [nchan] replacing out_scale, or null.
 cudaError_t launch_fstage(const Job &job, const float2 *twiddles, int t0, int nt, int T, void *chan, int chan_type,
@@ -93,13 +102,14 @@ cudaError_t fstage_tc32_take_error(int *flag);
 // xstage_fp32.cu: accumulates visibilities of FFTs [0, nt) of the block into
 // the compensated (sum, comp) accumulators in the output layout.
 cudaError_t launch_xstage_cuda_core(const void *chan, int chan_type, int nant, int nchan, int T, int nt, int autos,
-                                    const int2 *pairs, float2 *vsum, float2 *vcomp, cudaStream_t s);
+                                    const int2 *pairs, float2 *vsum, float2 *vcomp, cudaStream_t s,
+                                    bool first = false);
 // Device table of (J, K) 2-antenna tile pairs, J <= K, J-major (cudaMalloc'd; caller frees).
 cudaError_t make_tile_pairs(int nant, int2 **out);
 
 cudaError_t launch_xstage_cuda_core_pairs(const void *chan, int chan_type, int nant, int nchan, int T, int nt,
                                           int autos, const int2 *pairs, float2 *vsum, float2 *vcomp,
-                                          cudaStream_t s);
+                                          cudaStream_t s, bool first = false);
 
 // xstage_tc.cu: tcgen05 tensor-core X-stage over FP16 channelised data.
 // FP16 data: kind::f16 MMAs; FP32 data: kind::tf32 MMAs on a hi/lo split (FP32-accurate products).
@@ -108,10 +118,14 @@ cudaError_t launch_xstage_cuda_core_pairs(const void *chan, int chan_type, int n
 // kparts_max = 2 with plane > 0: the FP16 / FP8 kernel splits the block's FFTs across two CTAs
 // per channel group when the groups are fewer than the SMs (3: whenever the block is long enough),
 // the second CTA accumulating into vsum/vcomp + plane (a second plane the caller allocated, zeroed
-// and sums at the end).
+// where xstage_tensor_uses_plane says so, and sums at the end).
+// first (both engines): the accumulators hold nothing yet; the block's sums are stored (compensation 0) instead of added,
+// so they need no clearing.
 cudaError_t launch_xstage_tensor(const void *chan, int chan_type, int nant, int nchan, int T, int nt, int autos,
                                  float2 *vsum, float2 *vcomp, cudaStream_t s, int split_e = -1,
-                                 int kparts_max = 1, size_t plane = 0);
+                                 int kparts_max = 1, size_t plane = 0, bool first = false);
+// True when a block of nt FFTs puts sums into the second plane.
+int xstage_tensor_uses_plane(int nant, int nchan, int chan_type, int nt, int kparts_max);
 int xstage_tensor_supported(int nant);
 int xstage_tensor_channels_per_cta(int nant, int chan_type);
 int xstage_tensor_fits(int nant, int nchan, int chan_type);
@@ -129,6 +143,33 @@ gxc_status process_chained(gxc_handle *h, void *stream, cudaEvent_t copy_wait, c
 __host__ __device__ inline int baseline_index(int j, int k, int nant) {
   if (j == k) return nant * (nant - 1) / 2 + j;
   return j * nant - j * (j + 1) / 2 + (k - j - 1);
+}
+
+// Antennas of output baseline bl (the inverse of baseline_index).
+__device__ inline void baseline_antennas(int bl, int nant, int *j, int *k) {
+  const int ncross = nant * (nant - 1) / 2;
+  if (bl >= ncross) {
+    *j = *k = bl - ncross;
+    return;
+  }
+  int a = 0, rem = bl;
+  while (rem >= nant - 1 - a) {
+    rem -= nant - 1 - a;
+    a++;
+  }
+  *j = a;
+  *k = a + 1 + rem;
+}
+
+// Sum of c over the 256 threads of a block, returned to thread 0.
+__device__ inline int block_sum256(int c) {
+  __shared__ int red[8];
+  for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = c;
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int w = 1; w < 8; w++) c += red[w];
+  return c;
 }
 
 // Compensated accumulation acc += x (TwoSum): sum holds the running total,

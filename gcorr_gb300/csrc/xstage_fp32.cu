@@ -34,7 +34,7 @@ __device__ __forceinline__ void cmac_conj(float2 &a, float2 x, float2 y) {
 template <typename InT>
 __global__ void xstage_cc_kernel(const InT *__restrict__ chan, int nant, int nchan, int T, int nt, int autos,
                                  const int2 *__restrict__ tile_pairs, int npairs, int pairs_per_cta, int TT,
-                                 float2 *__restrict__ vsum, float2 *__restrict__ vcomp) {
+                                 float2 *__restrict__ vsum, float2 *__restrict__ vcomp, int first) {
   extern __shared__ unsigned char xsm_raw[];
   InT *xs = reinterpret_cast<InT *>(xsm_raw);  // [TT][nstream][CW]
   const int nstream = 2 * nant;
@@ -112,7 +112,11 @@ __global__ void xstage_cc_kernel(const InT *__restrict__ chan, int nant, int nch
 #pragma unroll
       for (int p = 0; p < 4; p++) {
         const size_t o = ((size_t)bl * 4 + p) * nchan + cg;
-        float2 s = vsum[o], e = vcomp[o];
+        float2 s = make_float2(0.f, 0.f), e = s;
+        if (!first) {
+          s = vsum[o];
+          e = vcomp[o];
+        }
         two_sum_add(s.x, e.x, acc[a][b][p].x);
         two_sum_add(s.y, e.y, acc[a][b][p].y);
         vsum[o] = s;
@@ -135,15 +139,15 @@ cudaError_t make_tile_pairs(int nant, int2 **out) {
 }
 
 cudaError_t launch_xstage_cuda_core(const void *chan, int chan_type, int nant, int nchan, int T, int nt, int autos,
-                                    const int2 *pairs, float2 *vsum, float2 *vcomp, cudaStream_t s) {
-  return launch_xstage_cuda_core_pairs(chan, chan_type, nant, nchan, T, nt, autos, pairs, vsum, vcomp, s);
+                                    const int2 *pairs, float2 *vsum, float2 *vcomp, cudaStream_t s, bool first) {
+  return launch_xstage_cuda_core_pairs(chan, chan_type, nant, nchan, T, nt, autos, pairs, vsum, vcomp, s, first);
 }
 
 // Same launch with a caller-provided tile-pair table (J <= K over ceil(nant/2)
 // antenna tiles, J-major), for callers that keep the table in their own memory.
 cudaError_t launch_xstage_cuda_core_pairs(const void *chan, int chan_type, int nant, int nchan, int T, int nt,
                                           int autos, const int2 *pairs, float2 *vsum, float2 *vcomp,
-                                          cudaStream_t s) {
+                                          cudaStream_t s, bool first) {
   if (nt <= 0) return cudaSuccess;
   const int nat = (nant + 1) / 2;
   const int npairs = nat * (nat + 1) / 2;
@@ -162,19 +166,19 @@ cudaError_t launch_xstage_cuda_core_pairs(const void *chan, int chan_type, int n
     e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     k<<<grid, threads, smem, s>>>((const float2 *)chan, nant, nchan, T, nt, autos, pairs, npairs, pairs_per_cta, TT,
-                                   vsum, vcomp);
+                                   vsum, vcomp, first);
   } else if (chan_type == CHAN_F8) {
     auto k = xstage_cc_kernel<__nv_fp8x2_e4m3>;
     e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     k<<<grid, threads, smem, s>>>((const __nv_fp8x2_e4m3 *)chan, nant, nchan, T, nt, autos, pairs, npairs,
-                                   pairs_per_cta, TT, vsum, vcomp);
+                                   pairs_per_cta, TT, vsum, vcomp, first);
   } else {
     auto k = xstage_cc_kernel<__half2>;
     e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     k<<<grid, threads, smem, s>>>((const __half2 *)chan, nant, nchan, T, nt, autos, pairs, npairs, pairs_per_cta, TT,
-                                   vsum, vcomp);
+                                   vsum, vcomp, first);
   }
   return cudaGetLastError();
 }

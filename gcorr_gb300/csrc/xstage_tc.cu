@@ -79,6 +79,7 @@ struct Params {
   // accumulating into plane `part` of vsum/vcomp (planes `plane` elements apart)
   int kparts, kspan;
   size_t plane;
+  int first;  // store the block's first-plane sums instead of adding them (the accumulators hold nothing yet)
   // FP16 / FP8 kernel: persist = 1 runs one CTA per SM over equal shares of all (group, chunk)
   // units; ngrp = channel groups of the launch
   int persist, ngrp;
@@ -88,9 +89,19 @@ struct Params {
 // use[i].  All loads of the batch are issued before its first store, so their latencies overlap
 // (one load-add-store at a time waited a full memory round trip per output: in the FP16
 // X-stage that was about a quarter of each CTA's time).
+// first: stores val[i] with compensation 0 instead (the accumulators hold nothing yet).
 template <int N>
 __device__ __forceinline__ void rmw_batch(float2 *vsum, float2 *vcomp, const size_t (&off)[N],
-                                          const float2 (&val)[N], const bool (&use)[N]) {
+                                          const float2 (&val)[N], const bool (&use)[N], bool first) {
+  if (first) {
+#pragma unroll
+    for (int i = 0; i < N; i++)
+      if (use[i]) {
+        vsum[off[i]] = val[i];
+        vcomp[off[i]] = make_float2(0.f, 0.f);
+      }
+    return;
+  }
   float2 sm[N], e[N];
 #pragma unroll
   for (int i = 0; i < N; i++)
@@ -456,7 +467,7 @@ __global__ void __launch_bounds__(NTHREADS_TC, 1) xstage_tc_kernel(Params p, con
               off[u] = (size_t)(e >> lcs) * p.nchan + cb + (e & (p.CS - 1));
               val[u] = use[u] ? stg[e] : make_float2(0.f, 0.f);
             }
-            rmw_batch<8>(vsum, vcomp, off, val, use);
+            rmw_batch<8>(vsum, vcomp, off, val, use, p.first && k0 == 0);
           }
         }
         mbar_arrive(smem_u32(&bar_stg[1]));
@@ -865,7 +876,7 @@ __global__ void __launch_bounds__(NTHREADS_SPLIT, 1) xstage_tc_split_kernel(Para
         off[u] = (size_t)(e >> lcs) * p.nchan + cb + (e & (p.CS - 1));
         val[u] = use[u] ? stg[e] : make_float2(0.f, 0.f);
       }
-      rmw_batch<8>(p.vsum, p.vcomp, off, val, use);
+      rmw_batch<8>(p.vsum, p.vcomp, off, val, use, p.first);
     }
   }
   if (warp == NPROD_WARPS) tmem_dealloc(tmem, TMEM_COLS);
@@ -1046,7 +1057,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) xstage_tc_big_kernel(Params p) {
             }
             const int bl = baseline_index(j, k, p.nant);
             const size_t o = ((size_t)bl * 4 + 2 * l + m) * p.nchan + c;
-            float2 sm = p.vsum[o], e = p.vcomp[o];
+            float2 sm = make_float2(0.f, 0.f), e = sm;
+            if (!p.first) {
+              sm = p.vsum[o];
+              e = p.vcomp[o];
+            }
             two_sum_add(sm.x, e.x, re);
             two_sum_add(sm.y, e.y, im);
             p.vsum[o] = sm;
@@ -1338,7 +1353,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) xstage_tc_big2_kernel(Params p) {
         off[u] = ((size_t)bl * 4 + prod) * p.nchan + c0 + ci;
         val[u] = use[u] ? stg[e] : make_float2(0.f, 0.f);
       }
-      rmw_batch<4>(p.vsum, p.vcomp, off, val, use);
+      rmw_batch<4>(p.vsum, p.vcomp, off, val, use, p.first);
     }
   }
   if (warp == NPROD_WARPS) tmem_dealloc(tmem, 512);
@@ -1431,9 +1446,27 @@ int xstage_tensor_fits(int nant, int nchan, int chan_type) {
   return cs > 0 && nchan % cs == 0;
 }
 
+// The block's FFTs go to two CTAs per channel group (see launch_xstage_tensor).
+static bool splits_block(int ngrp, int nsm, int nt, int KC, int kparts_max) {
+  return kparts_max >= 2 && nt >= 4 * KC && (ngrp < nsm || kparts_max >= 3);
+}
+
+int xstage_tensor_uses_plane(int nant, int nchan, int chan_type, int nt, int kparts_max) {
+  if (chan_type == CHAN_F32 || 4 * nant > 128 || kparts_max < 2) return 0;
+  int dev = 0, nsm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return 1;
+  const int KC = chan_type == CHAN_F8 ? 128 : tc::Cfg<false>::KC;
+  const int ngrp = nchan / xstage_tensor_channels_per_cta(nant, chan_type);
+  if (splits_block(ngrp, nsm, nt, KC, kparts_max)) return 1;
+  // persistent schedule: the last round's groups are halved when they are at most half the SMs (xstage_seg)
+  return kparts_max == 2 && ngrp >= nsm && ngrp % nsm != 0 && 2 * (ngrp % nsm) <= nsm && nt > KC;
+}
+
 cudaError_t launch_xstage_tensor(const void *chan, int chan_type, int nant, int nchan, int T, int nt, int autos,
                                  float2 *vsum, float2 *vcomp, cudaStream_t s, int split_e, int kparts_max,
-                                 size_t plane) {
+                                 size_t plane, bool first) {
   if (nt <= 0) return cudaSuccess;
   if (!xstage_tensor_supported(nant)) return cudaErrorInvalidValue;
   tc::Params p;
@@ -1457,6 +1490,7 @@ cudaError_t launch_xstage_tensor(const void *chan, int chan_type, int nant, int 
   p.ngrp = 0;
   p.kspan = nt;
   p.plane = plane;
+  p.first = first;
   // FP32 data: FP16 hi/lo split of values scaled by 2^-split_e when split_e >= 0, else TF32 split
   const bool h16 = chan_type == CHAN_F32 && split_e >= 0;
   p.split_sc = h16 ? ldexpf(1.0f, -split_e) : 1.0f;
@@ -1550,7 +1584,7 @@ cudaError_t launch_xstage_tensor(const void *chan, int chan_type, int nant, int 
     if (e != cudaSuccess) return e;
     p.ngrp = ngrp;
     p.persist = 0;
-    if (kparts_max >= 2 && plane > 0 && nt >= 4 * KC && (ngrp < nsm || kparts_max >= 3)) {
+    if (plane > 0 && splits_block(ngrp, nsm, nt, KC, kparts_max)) {
       p.kparts = 2;
       p.kspan = (nt / 2 + KC - 1) / KC * KC;
     } else if (kparts_max == 2 && plane > 0 && ngrp >= nsm) {
