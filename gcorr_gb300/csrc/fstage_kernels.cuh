@@ -141,7 +141,7 @@ struct FParams {
   const float2 *tw;    // W_F^m, m < F
   const float2 *twp1;  // F = 8192: pass-1 twiddles of the packed-pair kernel (make_twiddles), else null
   const float2 *twp2;  // F = 8192: pass-2 twiddles of the packed-pair kernel, else null
-  int t0, T;
+  int t0, nt, T;
   void *chan;
   float out_scale;
   int sub_shift, sub_mask;    // substride = 1 << sub_shift
@@ -170,7 +170,7 @@ inline int fparams_ilog2(int x) {
 }
 
 // Launch parameters of FFTs [t0, t0 + nt) of a block of T (twiddles from make_twiddles).
-inline FParams fstage_params(const Job &job, const float2 *twiddles, int t0, int T, void *chan, float out_scale,
+inline FParams fstage_params(const Job &job, const float2 *twiddles, int t0, int nt, int T, void *chan, float out_scale,
                              float2 *probe, const float *cscale = nullptr) {
   FParams prm;
   prm.job = job;
@@ -178,6 +178,7 @@ inline FParams fstage_params(const Job &job, const float2 *twiddles, int t0, int
   prm.twp1 = job.F == 8192 ? twiddles + job.F : nullptr;
   prm.twp2 = job.F == 8192 ? twiddles + job.F + kPairTw1 : nullptr;
   prm.t0 = t0;
+  prm.nt = nt;
   prm.T = T;
   prm.chan = chan;
   prm.out_scale = out_scale;
@@ -232,20 +233,27 @@ constexpr int hibit(int r) { return r >= 16 ? 16 : r >= 8 ? 8 : r >= 4 ? 4 : r >
 constexpr int log2c(int x) { return x <= 1 ? 0 : 1 + log2c(x / 2); }
 
 // Radix schedule and compile-time table splits for FFT length 2^L.
-// A CTA transforms one pol of one FFT window; each of its F/32 threads holds
-// 32 complex values per pass (2 or 3 passes, radices <= 32); two CTAs share an SM.
+// F/32 threads hold 32 complex values per pass (2 or 3 passes, radices <= 32) of one pol of one window; the kernel is
+// bound by instruction issue.  Up to 4096 points a CTA transforms both pols of a window, which share the staged bytes and
+// the rotator and frac-delay tables; at 256 points two windows fill its warp.  With one pol per CTA every table entry
+// was evaluated twice, 16 of 32 lanes worked at 512 points and 8 at 256, and few CTAs were resident: 7 antennas of
+// 512-point complex windows, 32003 FFTs, FP16 output, took 0.89 ms and now take 0.45 ms.  Above 4096 points a CTA of two
+// pols would need 512 threads of 128 registers, all of an SM, and nothing would cover its barriers.
 template <int L, bool CPLX>
 struct FPlan {
   static constexpr int N = 1 << L;
-  static constexpr int NTW = N / 32;                  // threads with FFT work
-  static constexpr int NT = NTW < 32 ? 32 : NTW;      // threads launched
+  static constexpr int NTW = N / 32;                  // threads per transform
+  static constexpr int NPOL = L <= 12 ? 2 : 1;        // pols per CTA
+  static constexpr int NWIN = L == 8 ? 2 : 1;         // windows per CTA
+  static constexpr int NT = NTW * NPOL * NWIN;        // threads launched
   static constexpr int R0 = L == 8 ? 16 : L == 9 ? 32 : L == 10 ? 32 : L == 11 ? 8 : L == 12 ? 16 : L == 13 ? 32 : 16;
   static constexpr int R1 = L == 8 ? 16 : L == 9 ? 16 : L == 10 ? 32 : L == 14 ? 32 : 16;
   static constexpr int R2 = L <= 10 ? 1 : (L == 14 ? 32 : 16);
   static constexpr int RL = R2 > 1 ? R2 : R1;         // radix of the last pass
   static constexpr int PAD = R0;                      // one smem slot of padding per R0 (conflict-free strided stores)
   static constexpr int PADN = N + N / R0;
-  static constexpr int MINB = (L >= 14) ? 1 : 2;      // CTAs per SM (F = 16384 fills the shared memory)
+  // CTAs per SM at 128 registers per thread (F = 16384 fills the shared memory)
+  static constexpr int MINB = L >= 14 ? 1 : 512 / NT;
   // table splits, fxkernel.cpp:57-64 (stride = sqrt(nchan) for square nchan; 2^floor(log2(nchan)/2) otherwise)
   static constexpr int NCHAN = CPLX ? N : N / 2;
   static constexpr int STRIDE = 1 << (log2c(NCHAN) / 2);
@@ -289,71 +297,83 @@ __global__ void __launch_bounds__(FPlan<L, CPLX>::NT, FPlan<L, CPLX>::MINB) fsta
   constexpr int N = Pl::N, NT = Pl::NT, NTW = Pl::NTW;
   constexpr int R0 = Pl::R0, R1 = Pl::R1, R2 = Pl::R2, RL = Pl::RL, PAD = Pl::PAD;
   constexpr int SUB = Pl::SUB, STRIDE = Pl::STRIDE, FSUB = Pl::FSUB, NCHAN = Pl::NCHAN;
+  constexpr int NPOL = Pl::NPOL, NWIN = Pl::NWIN;
   const Job &job = prm.job;
   extern __shared__ float2 smem[];
-  float2 *buf = smem;                     // N + N/R0 (padded)
-  float2 *tsub = buf + Pl::PADN;          // fringe rotator, fine part  [SUB]
-  float2 *tstep = tsub + SUB;             // fringe rotator, coarse part [STRIDE]
-  float2 *fsubt = tstep + STRIDE;         // frac-delay, fine part [FSUB]
-  float2 *fstept = fsubt + FSUB;          // frac-delay, coarse part [STRIDE]
-  unsigned char *stage = reinterpret_cast<unsigned char *>(fstept + STRIDE);  // packed input window
+  // per transform: N + N/R0 slots (padded); per window: the tables, then the packed input window
+  constexpr int TABS = SUB + 2 * STRIDE + FSUB;
+  constexpr int STAGE = ((CPLX ? 4 * N + 32 : N / 2 + 32) + 15) & ~15;
+  const int tid = threadIdx.x;
+  const int unit = tid / NTW, ut = tid - unit * NTW;  // transform of this thread, thread of the transform
+  const int wsub = unit / NPOL;                       // window of the CTA
+  float2 *buf = smem + unit * Pl::PADN;
+  float2 *tsub = smem + NPOL * NWIN * Pl::PADN + wsub * TABS;  // fringe rotator, fine part  [SUB]
+  float2 *tstep = tsub + SUB;                                  // fringe rotator, coarse part [STRIDE]
+  float2 *fsubt = tstep + STRIDE;                              // frac-delay, fine part [FSUB]
+  float2 *fstept = fsubt + FSUB;                               // frac-delay, coarse part [STRIDE]
+  unsigned char *stage =
+      reinterpret_cast<unsigned char *>(smem + NPOL * NWIN * Pl::PADN + NWIN * TABS) + wsub * STAGE;
 
-  // grid x = pol + 2 * FFT: the two pols of one window run side by side (the second
-  // read of the packed window hits L2) and write neighbouring streams
-  const int pol = blockIdx.x & 1;  // the pol this CTA transforms
-  const int tl = blockIdx.x >> 1;
+  // grid x = FFT (and the pol, one pol per CTA: the two pols of one window run side by side, and the second read of the
+  // packed window hits L2)
+  const int pol = NPOL == 2 ? unit & 1 : blockIdx.x & 1;
+  const int tl = NPOL == 2 ? blockIdx.x * NWIN + wsub : blockIdx.x >> 1;
   const int ant = blockIdx.y;
   const int t = prm.t0 + tl;
-  const int tid = threadIdx.x;
+  const bool exists = NWIN == 1 || tl < prm.nt;
   const int nstreams = 2 * job.nant;
   const int s = 2 * ant + pol;
   OutT *chan = reinterpret_cast<OutT *>(prm.chan);
   // every thread reads the 32-byte record (one broadcast load): no barrier needed
-  const Geom g = job.geom[(size_t)ant * job.nfft + t];
+  Geom g = job.geom[(size_t)ant * job.nfft + (exists ? t : prm.t0)];
+  if (!exists) g.valid = 0;
 
   // channelised layout [ctile][t][stream][16]: element (c, s) of this FFT
   OutT *out0 = chan + ((size_t)tl * nstreams + s) * CW;
   const size_t ctile_stride = (size_t)prm.T * nstreams * CW;
 
-  if (!g.valid) {
+  if (!g.valid && exists) {
     // flagged: the X-stage sums zeros, the baseline counts exclude this FFT
     const OutT z = to_out<OutT>(make_float2(0.f, 0.f), 1.f);
-    for (int c = tid; c < NCHAN; c += NT) out0[(size_t)(c >> 4) * ctile_stride + (c & 15)] = z;
-    return;
+    for (int c = ut; c < NCHAN; c += NTW) out0[(size_t)(c >> 4) * ctile_stride + (c & 15)] = z;
   }
+  if (NWIN == 1 && !g.valid) return;
 
   const long long stage_base = (CPLX ? 4LL * g.offset : ((long long)g.offset >> 1)) & ~15LL;
-  {
+  if (g.valid) {
     // stage the packed window with 16-byte loads (bounds: the buffer holds
     // (nfft+1)*F samples and offset <= (nfft-1)*F, so the window plus the
     // 16-byte rounding stays inside it)
+    const int wt = tid - wsub * (NPOL * NTW);  // thread of the window
+    constexpr int WT = NPOL * NTW;
     const uint4 *src = reinterpret_cast<const uint4 *>(job.inputs[ant] + stage_base);
     const long long last = CPLX ? 4LL * (g.offset + N) : (((long long)g.offset + N + 1) >> 1);
     const int nvec = (int)((last - stage_base + 15) >> 4);
     uint4 *dst = reinterpret_cast<uint4 *>(stage);
-    for (int i = tid; i < nvec; i += NT) dst[i] = __ldg(&src[i]);
+    for (int i = wt; i < nvec; i += WT) cp_async16(dst + i, src + i);
     const float c0 = g.c0, c1 = g.c1, cstep = g.cstep, cf = g.cf;
-    for (int k = tid; k < SUB; k += NT) {
+    for (int k = wt; k < SUB; k += WT) {
       float sn, cs;
       sincospif(-2.0f * fmaf((float)k, c1, c0), &sn, &cs);
       tsub[k] = make_float2(cs, sn);
     }
-    for (int i = tid; i < STRIDE; i += NT) {
+    for (int i = wt; i < STRIDE; i += WT) {
       float sn, cs;
       sincospif(-2.0f * ((float)i * cstep), &sn, &cs);
       tstep[i] = make_float2(cs, sn);
       sincospif(2.0f * ((float)(i * FSUB) * cf), &sn, &cs);
       fstept[i] = make_float2(cs, sn);
     }
-    for (int k = tid; k < FSUB; k += NT) {
+    for (int k = wt; k < FSUB; k += WT) {
       float sn, cs;
       sincospif(2.0f * ((float)k * cf), &sn, &cs);
       fsubt[k] = make_float2(cs, sn);
     }
+    cp_async_wait_all();
   }
   __syncthreads();
 
-  const bool active = tid < NTW;
+  const bool active = g.valid;
   const int off = g.offset;
   float2 u[32];
   // ---- pass 0 (span 1): decode + fringe-rotate from the staged window
@@ -362,7 +382,7 @@ __global__ void __launch_bounds__(FPlan<L, CPLX>::NT, FPlan<L, CPLX>::MINB) fsta
     const int sbase = (int)(CPLX ? (4LL * off - stage_base) : (((long long)off >> 1) - stage_base));
 #pragma unroll
     for (int q = 0; q < 32 / R0; q++) {
-      const int iv = tid + q * NTW;
+      const int iv = ut + q * NTW;
       float2 *v = &u[q * R0];
       // this thread's samples n = iv + r*NB: fine rotator index fixed, coarse index strided
       const float2 rs = tsub[iv & (SUB - 1)];
@@ -395,7 +415,7 @@ __global__ void __launch_bounds__(FPlan<L, CPLX>::NT, FPlan<L, CPLX>::MINB) fsta
   if (active) {
 #pragma unroll
     for (int q = 0; q < 32 / R0; q++) {
-      const int iv = tid + q * NTW;
+      const int iv = ut + q * NTW;
       float2 *b = buf + iv * (R0 + 1);
 #pragma unroll
       for (int r = 0; r < R0; r++) b[r] = u[q * R0 + r];
@@ -409,7 +429,7 @@ __global__ void __launch_bounds__(FPlan<L, CPLX>::NT, FPlan<L, CPLX>::MINB) fsta
     if (active) {
 #pragma unroll
       for (int q = 0; q < 32 / R1; q++) {
-        const int iv = tid + q * NTW;
+        const int iv = ut + q * NTW;
         const float2 *b = buf + iv + iv / PAD;
 #pragma unroll
         for (int r = 0; r < R1; r++) u[q * R1 + r] = b[r * (NB + NB / PAD)];
@@ -421,7 +441,7 @@ __global__ void __launch_bounds__(FPlan<L, CPLX>::NT, FPlan<L, CPLX>::MINB) fsta
     if (active) {
 #pragma unroll
       for (int q = 0; q < 32 / R1; q++) {
-        const int iv = tid + q * NTW;
+        const int iv = ut + q * NTW;
         const int k = iv & (R0 - 1);
         const int j = (iv - k) * R1 + k;
         float2 *b = buf + j + j / PAD;
@@ -439,7 +459,7 @@ __global__ void __launch_bounds__(FPlan<L, CPLX>::NT, FPlan<L, CPLX>::MINB) fsta
     constexpr int RKEEP = CPLX ? RL : RL / 2;  // real data keeps channels c < N/2
 #pragma unroll
     for (int q = 0; q < 32 / RL; q++) {
-      const int iv = tid + q * NTW;
+      const int iv = ut + q * NTW;
       float2 *v = &u[q * RL];
       const float2 *b = buf + iv + iv / PAD;
 #pragma unroll
@@ -795,12 +815,14 @@ static cudaError_t launch_fstage_t(const FParams &prm, int nt, cudaStream_t s) {
       job.nchan != Pl::NCHAN)
     return cudaErrorInvalidValue;
   const size_t stage_bytes = CPLX ? 4 * (size_t)Pl::N + 32 : (size_t)Pl::N / 2 + 32;
-  const size_t smem = sizeof(float2) * ((size_t)Pl::PADN + Pl::SUB + 2 * Pl::STRIDE + Pl::FSUB) +
-                      ((stage_bytes + 15) & ~(size_t)15);
+  const size_t smem = sizeof(float2) * ((size_t)Pl::NPOL * Pl::NWIN * Pl::PADN +
+                                        (size_t)Pl::NWIN * (Pl::SUB + 2 * Pl::STRIDE + Pl::FSUB)) +
+                      Pl::NWIN * ((stage_bytes + 15) & ~(size_t)15);
   auto kern = fstage_kernel<L, OutT, CPLX, DBG>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  dim3 grid(2u * (unsigned)nt, (unsigned)job.nant, 1u);
+  const unsigned nx = Pl::NPOL == 2 ? ((unsigned)nt + Pl::NWIN - 1) / Pl::NWIN : 2u * (unsigned)nt;
+  dim3 grid(nx, (unsigned)job.nant, 1u);
   kern<<<grid, Pl::NT, smem, s>>>(prm);
   return cudaGetLastError();
 }

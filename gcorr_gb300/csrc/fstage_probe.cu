@@ -13,7 +13,7 @@ namespace gxc {
 cudaError_t launch_fstage_probe(const Job &job, const float2 *twiddles, int t0, int nt, int T, void *chan,
                                 int chan_type, float out_scale, float2 *probe, cudaStream_t s) {
   if (nt <= 0) return cudaSuccess;
-  const FParams prm = fstage_params(job, twiddles, t0, T, chan, out_scale, probe);
+  const FParams prm = fstage_params(job, twiddles, t0, nt, T, chan, out_scale, probe);
   // FP16 / FP8 output at 16384 and 32768 points runs the FP16-buffer kernel; every other
   // shape runs a kernel template whose decode does not depend on the output type, probed
   // here with FP32 output (chan must then hold T FFTs of FP32 channelised data)
