@@ -126,6 +126,13 @@ cudaError_t launch_xstage_tensor(const void *chan, int chan_type, int nant, int 
                                  int kparts_max = 1, size_t plane = 0, bool first = false);
 // True when a block of nt FFTs puts sums into the second plane.
 int xstage_tensor_uses_plane(int nant, int nchan, int chan_type, int nt, int kparts_max);
+// The X-stage over FP32 spectra where they are, ants [2 nant][nfft * fftwidth] (gxc_xcorr's layout): no channelised copy, no
+// accumulators, the sums of all nfft FFTs divided by nfft stored to out.  chan_type CHAN_F32 (TF32 split) or CHAN_F16
+// (values rounded to FP16); tensor maps want a 16-byte aligned base and an even fftwidth.
+constexpr int kDirectSpan = 1024;  // FFTs of one CTA; a cluster of up to 8 takes a channel group
+int xstage_direct_fits(const void *ants, int nant, int nfft, int nchan, int fftwidth, int chan_type);
+cudaError_t launch_xstage_direct(const void *ants, int chan_type, int nant, int nfft, int nchan, int fftwidth, int autos,
+                                 float2 *out, cudaStream_t s);
 int xstage_tensor_supported(int nant);
 int xstage_tensor_channels_per_cta(int nant, int chan_type);
 int xstage_tensor_fits(int nant, int nchan, int chan_type);

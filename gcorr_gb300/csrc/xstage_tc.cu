@@ -22,6 +22,7 @@
 // visibility accumulators.  The 33-64 antenna kernel loads with plain gathers.
 // Every mbarrier wait is bounded (iteration cap and %globaltimer); on expiry
 // the kernel raises an error flag, lets issued MMAs drain, frees TMEM and exits.
+#include <cooperative_groups.h>
 #include <cuda.h>
 #include <stdint.h>
 
@@ -83,6 +84,9 @@ struct Params {
   // FP16 / FP8 kernel: persist = 1 runs one CTA per SM over equal shares of all (group, chunk)
   // units; ngrp = channel groups of the launch
   int persist, ngrp;
+  // split kernel: kparts CTAs of a cluster (1: no cluster) take kspan FFTs each of one channel group; out not null: the
+  // results divided by the FFT count go there, and vsum / vcomp are not touched
+  float2 *out;
 };
 
 // Adds val[i] into the compensated accumulators (vsum, vcomp) at off[i], for every i < N with
@@ -544,10 +548,19 @@ constexpr int TMA_WARP_SPLIT = NPROD_WARPS + 1 + NEPI_WARPS;
 // values in FP16's normal range; a subnormal lo only adds an absolute error near 2^-25),
 // kind::f16 at twice the tf32 rate and half the shared-memory bytes, 64 FFTs per stage.  Used
 // where the data's scale is known (the F-stage's output): FP16's exponent range must hold it.
-template <int R, bool H16>
+//
+// FORM 0 is the TF32 split, 1 the FP16 split, both of the channelised layout.  Forms 2 and 3 read spectra as a caller holds
+// them, [stream][FFT][channel]: 3 is the TF32 split; 2 rounds to FP16 (the precision FP16 of data that arrives in FP32)
+// and needs no lo tile.  Their TMA boxes run through the FFTs of a stream before the next stream, since streams lie
+// megabytes apart: with the stream inside, every row of 16 to 128 bytes was in another page, and 16 antennas x 1024
+// channels x 2048 FFTs took 473 us a call, now 183.  The raw tile then is [stream][FFT][channels]; a warp's lanes take
+// different K chunks o of a stream, and each lane reads its FFTs in an order turned by a function of o, so that eight
+// lanes meet eight banks of 16 bytes.  The order within a K chunk is the same for every row, which a Gram sum allows.
+template <int R, int FORM>
 __global__ void __launch_bounds__(NTHREADS_SPLIT, 1) xstage_tc_split_kernel(Params p,
                                                                             const __grid_constant__ CUtensorMap tmap) {
   using C = Cfg<true>;
+  constexpr bool H16 = FORM == 1 || FORM == 2, LO = FORM != 2, DIRECT = FORM >= 2;
   constexpr int KC = H16 ? 64 : C::KC, KSTEP = H16 ? 16 : C::KSTEP;
   constexpr int TKC = H16 ? 8 : 4;       // FFTs per 16-byte chunk of an operand row
   constexpr int NG = C::NG, GROUP_BYTES = C::GROUP_BYTES, STAGE_BYTES = C::STAGE_BYTES;
@@ -565,9 +578,12 @@ __global__ void __launch_bounds__(NTHREADS_SPLIT, 1) xstage_tc_split_kernel(Para
   const uint32_t sbase = smem_u32(smem);
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
-  const int cb = blockIdx.x * p.CS;
+  const int part = (int)blockIdx.x % p.kparts;        // rank in the cluster
+  const int cb = ((int)blockIdx.x / p.kparts) * p.CS;
   const int n = p.nstream;
-  const int nchunks = (p.nt + KC - 1) / KC;
+  const int t0 = part * p.kspan;                      // first FFT of this CTA
+  const int ntp = p.nt - t0 < p.kspan ? p.nt - t0 : p.kspan;
+  const int nchunks = ntp > 0 ? (ntp + KC - 1) / KC : 0;
   const int nper = (nchunks + DP - 1) / DP;
 
   if (2 * n < R) {  // zero the padding rows of both tiles (hi, lo) of every group of every stage
@@ -624,8 +640,11 @@ __global__ void __launch_bounds__(NTHREADS_SPLIT, 1) xstage_tc_split_kernel(Para
         if (rc >= RSTAGES && !mbar_wait(smem_u32(&raw_empty[rs]), ((rc / RSTAGES) - 1) & 1, p.err)) break;
         const uint32_t bar = smem_u32(&raw_full[rs]);
         mbar_expect_tx(bar, (uint32_t)(p.rbox_bytes * p.rnbox));
-        for (int j = 0; j < p.rnbox; j++)
-          tma_load_4d(raw_s + rs * RAW_BYTES + j * p.rbox_bytes, &tmap, x0, 0, rc * KCR, (cb >> 4) + j, bar);
+        for (int j = 0; j < p.rnbox; j++) {
+          const int t = t0 + rc * KCR;
+          tma_load_4d(raw_s + rs * RAW_BYTES + j * p.rbox_bytes, &tmap, x0, DIRECT ? t : 0, DIRECT ? 0 : t, (cb >> 4) + j,
+                      bar);
+        }
         issued = rc + 1;
       }
       for (int rc = issued > RSTAGES ? issued - RSTAGES : 0; rc < issued; rc++)
@@ -642,14 +661,30 @@ __global__ void __launch_bounds__(NTHREADS_SPLIT, 1) xstage_tc_split_kernel(Para
     const int nq = p.CS / 2;           // channel pairs
     const int kq = KCR / TKC;          // 16-byte K chunks per raw chunk
     const int ntask = kq * n * nq;     // (pair, stream, K chunk) per raw chunk
-    const size_t tstride = (size_t)n * BX * 8;  // bytes between FFT rows of a box
+    const size_t tstride = (DIRECT ? (size_t)BX : (size_t)n * BX) * 8;  // bytes between FFT rows of a box
+    const size_t sstride = (DIRECT ? (size_t)KCR * BX : (size_t)BX) * 8;  // and between streams
     const float sc = p.split_sc;
     // A thread's tasks are the same in every raw chunk: tid and tid + NPROD (the launcher
     // keeps ntask <= 2 NPROD), decoded once here so the chunk loop does no integer division.
-    int tq[2], ts[2], to[2];
+    int tq[2], ts[2], to[2], tf[2];
 #pragma unroll
     for (int j = 0; j < 2; j++) {
       const int task = tid + j * NPROD;
+      if constexpr (DIRECT) {
+        // 16-byte unit of (o, FFT i, pair q) within 128 bytes: (TKC o nq + i nq + q) mod 8.  With eight K chunks (TF32) the
+        // bits of o go to q and then to the turn f of i; with four (FP16) lane bit 2 is q's lowest bit.
+        const int lnq = 31 - __clz(nq), rest = task / kq, o = task & (kq - 1), qi = rest & (nq - 1);
+        to[j] = o;
+        ts[j] = rest >> lnq;
+        if constexpr (TKC == 4) {
+          tq[j] = qi ^ (o & (nq - 1));
+          tf[j] = o >> (lnq ? lnq : 1);
+        } else {
+          tq[j] = qi ^ ((o << 1) & (nq - 1));
+          tf[j] = lnq > 1 ? o >> (lnq - 1) : o;
+        }
+        continue;
+      }
       const int rest = task / nq;
       tq[j] = task - rest * nq;
       to[j] = rest / n;
@@ -681,10 +716,11 @@ __global__ void __launch_bounds__(NTHREADS_SPLIT, 1) xstage_tc_split_kernel(Para
             const int q = tq[j0 + u2], s = ts[j0 + u2], o = to[j0 + u2];
             const int cc0 = cofs + 2 * q;
             const unsigned char *src =
-                raw + (cc0 >> 4) * boxb + ((size_t)(TKC * o) * n + s) * BX * 8 + (cc0 & 15) * 8;
+                raw + (cc0 >> 4) * boxb + (size_t)(TKC * o) * tstride + s * sstride + (cc0 & 15) * 8;
 #pragma unroll
             for (int i = 0; i < TKC; i++)
-              v[u2][i] = task < ntask ? *reinterpret_cast<const float4 *>(src + i * tstride)
+              v[u2][i] = task < ntask ? *reinterpret_cast<const float4 *>(
+                                            src + (DIRECT ? (i + tf[j0 + u2]) & (TKC - 1) : i) * tstride)
                                       : make_float4(0.f, 0.f, 0.f, 0.f);
           }
 #pragma unroll
@@ -695,7 +731,7 @@ __global__ void __launch_bounds__(NTHREADS_SPLIT, 1) xstage_tc_split_kernel(Para
             const int oo = rr * kq + o;  // K chunk within the 128-byte row
             // which part (re, im) this lane stores first: among 8 lanes the first stores
             // then cover all 8 swizzle positions (no bank conflicts)
-            const int sw = nq == 1 ? ((s >> 2) & 1) : (q & 1);
+            const int sw = DIRECT ? 0 : nq == 1 ? ((s >> 2) & 1) : (q & 1);
 #pragma unroll
             for (int ci = 0; ci < 2; ci++) {
               const int cc = 2 * q + ci;
@@ -714,10 +750,12 @@ __global__ void __launch_bounds__(NTHREADS_SPLIT, 1) xstage_tc_split_kernel(Para
                     // packed conversions (cvt.rn.f16x2.f32): the same round-to-nearest halves,
                     // two values and their packing per instruction
                     const __half2 h = __floats2half2_rn(x0v, x1v);
-                    const float2 hb = __half22float2(h);
-                    const __half2 lw = __floats2half2_rn(2.0f * (x0v - hb.x), 2.0f * (x1v - hb.y));
                     hi[i] = reinterpret_cast<const uint32_t &>(h);
-                    lo[i] = reinterpret_cast<const uint32_t &>(lw);
+                    if constexpr (LO) {
+                      const float2 hb = __half22float2(h);
+                      const __half2 lw = __floats2half2_rn(2.0f * (x0v - hb.x), 2.0f * (x1v - hb.y));
+                      lo[i] = reinterpret_cast<const uint32_t &>(lw);
+                    }
                   }
                 } else {
 #pragma unroll
@@ -731,8 +769,9 @@ __global__ void __launch_bounds__(NTHREADS_SPLIT, 1) xstage_tc_split_kernel(Para
                 unsigned char *gbase = stage + G * GROUP_BYTES;
                 const int swz = (oo ^ (row & 7)) << 4;
                 *reinterpret_cast<uint4 *>(gbase + row * 128 + swz) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                *reinterpret_cast<uint4 *>(gbase + TILE_BYTES + row * 128 + swz) =
-                    make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                if constexpr (LO)
+                  *reinterpret_cast<uint4 *>(gbase + TILE_BYTES + row * 128 + swz) =
+                      make_uint4(lo[0], lo[1], lo[2], lo[3]);
               }
             }
           }
@@ -765,7 +804,7 @@ __global__ void __launch_bounds__(NTHREADS_SPLIT, 1) xstage_tc_split_kernel(Para
             const uint64_t dl = desc_sw128(sa + G * GROUP_BYTES + TILE_BYTES + kk * 32);
             if constexpr (H16) {
               mma_f16(d, dh, dh, IDESC, (first && kk == 0) ? 0u : 1u);
-              mma_f16(d, dl, dh, IDESC, 1u);
+              if constexpr (LO) mma_f16(d, dl, dh, IDESC, 1u);
             } else {
               mma_tf32(d, dh, dh, IDESC_TF32, (first && kk == 0) ? 0u : 1u);
               mma_tf32(d, dl, dh, IDESC_TF32, 1u);
@@ -874,10 +913,36 @@ __global__ void __launch_bounds__(NTHREADS_SPLIT, 1) xstage_tc_split_kernel(Para
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (!*(volatile int *)p.err) {  // a timed-out role may have left the staging incomplete
-    const int nbl = p.nant * (p.nant - 1) / 2 + (p.autos ? p.nant : 0);
-    const int nent = nbl * 4 * p.CS;
-    const int lcs = 31 - __clz(p.CS);  // CS is a power of two
+  const int nbl = p.nant * (p.nant - 1) / 2 + (p.autos ? p.nant : 0);
+  const int nent = nbl * 4 * p.CS;
+  const int lcs = 31 - __clz(p.CS);  // CS is a power of two
+  if (p.out) {
+    // The parts' sums meet through distributed shared memory: every CTA of the cluster adds up its share of the entries,
+    // in the order of the FFTs and compensated.  All threads take both cluster barriers, whatever happened before.
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    if (p.kparts > 1) cluster.sync();
+    if (!*(volatile int *)p.err) {
+      const float nf = (float)p.nt;
+      for (int e = part * NTHREADS_SPLIT + tid; e < nent; e += p.kparts * NTHREADS_SPLIT) {
+        float2 sm = make_float2(0.f, 0.f), cm = sm;
+        for (int r = 0; r < p.kparts; r++) {
+          const float2 *src = reinterpret_cast<const float2 *>(smem);
+          if (p.kparts > 1) src = cluster.map_shared_rank(src, r);
+          const float2 x = src[e];
+          if (r == 0) {
+            sm = x;
+          } else {
+            two_sum_add(sm.x, cm.x, x.x);
+            two_sum_add(sm.y, cm.y, x.y);
+          }
+        }
+        p.out[(size_t)(e >> lcs) * p.nchan + cb + (e & (p.CS - 1))] =
+            make_float2((sm.x + cm.x) / nf, (sm.y + cm.y) / nf);
+      }
+    }
+    if (p.kparts > 1) cluster.sync();  // no CTA leaves while another reads its shared memory
+  } else if (!*(volatile int *)p.err) {  // a timed-out role may have left the staging incomplete
     const float2 *stg = reinterpret_cast<const float2 *>(smem);
     for (int e0 = tid; e0 < nent; e0 += 8 * NTHREADS_SPLIT) {
       size_t off[8];
@@ -1425,21 +1490,21 @@ static EncodeTiledFn encode_tiled() {
   return fn;
 }
 
-// Tensor map of the channelised block [ctile][T][n][16] (esz bytes per complex value) for the
-// raw TMA tiles of the small-N tensor kernels: dims (channel in tile, stream, FFT, tile), the
-// FFT extent cut at nt so rows of later FFTs read as zeros; box (bx, n, kc, 1).
-static cudaError_t raw_tensor_map(CUtensorMap *m, const void *chan, int esz, int n, int nt, int T, int nchan, int bx,
-                                  int kc) {
+// Tensor map of complex data (esz bytes each) for the raw TMA tiles of the small-N tensor kernels: dims (channel in
+// tile, two of n0 and n1 entries stride0 and stride1 bytes apart, tile), box (bx, b0, b1, 1); what lies past an extent
+// reads as zeros.
+static cudaError_t raw_tensor_map(CUtensorMap *m, const void *data, int esz, int nchan, int bx, int n0, size_t stride0,
+                                  int b0, int n1, size_t stride1, int b1, size_t tile_stride) {
   EncodeTiledFn fn = encode_tiled();
   if (!fn) return cudaErrorNotSupported;
   const CUtensorMapDataType dt = esz == 8   ? CU_TENSOR_MAP_DATA_TYPE_INT64
                                  : esz == 4 ? CU_TENSOR_MAP_DATA_TYPE_UINT32
                                             : CU_TENSOR_MAP_DATA_TYPE_UINT16;
-  const cuuint64_t dims[4] = {(cuuint64_t)CW, (cuuint64_t)n, (cuuint64_t)nt, (cuuint64_t)(nchan / CW)};
-  const cuuint64_t strides[3] = {(cuuint64_t)CW * esz, (cuuint64_t)CW * n * esz, (cuuint64_t)CW * n * T * esz};
-  const cuuint32_t box[4] = {(cuuint32_t)bx, (cuuint32_t)n, (cuuint32_t)kc, 1u};
+  const cuuint64_t dims[4] = {(cuuint64_t)CW, (cuuint64_t)n0, (cuuint64_t)n1, (cuuint64_t)(nchan / CW)};
+  const cuuint64_t strides[3] = {(cuuint64_t)stride0, (cuuint64_t)stride1, (cuuint64_t)tile_stride};
+  const cuuint32_t box[4] = {(cuuint32_t)bx, (cuuint32_t)b0, (cuuint32_t)b1, 1u};
   const cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
-  const CUresult r = fn(m, dt, 4, const_cast<void *>(chan), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  const CUresult r = fn(m, dt, 4, const_cast<void *>(data), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                         CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
@@ -1478,6 +1543,89 @@ int xstage_tensor_uses_plane(int nant, int nchan, int chan_type, int nt, int kpa
   return kparts_max == 2 && ngrp >= nsm && ngrp % nsm != 0 && 2 * (ngrp % nsm) <= nsm && nt > KC;
 }
 
+// The split kernel for R rows per channel block: p.kparts CTAs (a cluster) per channel group.
+template <int FORM>
+static cudaError_t launch_split(int R, const tc::Params &p, const CUtensorMap &tmap, size_t smem, cudaStream_t s) {
+  auto run = [&](auto kern) -> cudaError_t {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(p.nchan / p.CS * p.kparts));
+    cfg.blockDim = dim3(tc::NTHREADS_SPLIT);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)p.kparts;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = p.kparts > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, p, tmap);
+  };
+  switch (R) {
+    case 16: return run(tc::xstage_tc_split_kernel<16, FORM>);
+    case 32: return run(tc::xstage_tc_split_kernel<32, FORM>);
+    case 64: return run(tc::xstage_tc_split_kernel<64, FORM>);
+    case 128: return run(tc::xstage_tc_split_kernel<128, FORM>);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+constexpr size_t kSplitSmem = (size_t)tc::STAGES * 65536 + (size_t)tc::RSTAGES * tc::RAW_BYTES + 1024;
+
+int xstage_direct_fits(const void *ants, int nant, int nfft, int nchan, int fftwidth, int chan_type) {
+  if (chan_type == CHAN_F8 || nant < 1 || 4 * nant > 128 || nfft > 8 * kDirectSpan) return 0;
+  if (!xstage_tensor_fits(nant, nchan, CHAN_F32)) return 0;
+  return ((uintptr_t)ants & 15) == 0 && fftwidth % 2 == 0 && (unsigned long long)nfft * fftwidth * 8 < (1ull << 40);
+}
+
+cudaError_t launch_xstage_direct(const void *ants, int chan_type, int nant, int nfft, int nchan, int fftwidth, int autos,
+                                 float2 *out, cudaStream_t s) {
+  if (!xstage_direct_fits(ants, nant, nfft, nchan, fftwidth, chan_type)) return cudaErrorInvalidValue;
+  tc::Params p = {};
+  p.chan = ants;
+  p.nant = nant;
+  p.nstream = 2 * nant;
+  p.nchan = nchan;
+  p.T = p.nt = nfft;
+  p.autos = autos;
+  p.R = 16;
+  while (p.R < 2 * p.nstream) p.R <<= 1;
+  p.g = 128 / p.R;
+  p.CS = xstage_tensor_channels_per_cta(nant, CHAN_F32);
+  p.split_sc = p.split_unsc = 1.0f;
+  p.out = out;
+  const bool f16 = chan_type == CHAN_F16;
+  const int KC = f16 ? 64 : tc::Cfg<true>::KC;
+  // A raw tile of 32 FFTs is at most 32 KiB (CS <= 64 / nant channels, to the power of two below), an operand stage the
+  // TF32 form's whole K extent or half the FP16 form's; at most two tasks per producer thread.  The staged results,
+  // [baseline x product][CS], fit the operand ring: at most 528 x 4 x 2 values (32 antennas).
+  static_assert(64 * 2 * 32 * 8 <= tc::RAW_BYTES && 528 * 4 * 2 * 8 <= tc::STAGES * 65536, "direct tiles");
+  p.rnbox = 1;
+  p.rbx = p.CS;
+  p.rkc = 32;
+  p.rbox_bytes = p.CS * p.nstream * 32 * 8;
+  if (p.CS < 2 || p.CS > CW || p.rbox_bytes > tc::RAW_BYTES) return cudaErrorInvalidValue;
+  int dev = 0, nsm = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess) e = xstage_tensor_error_flag(&p.err);
+  if (e != cudaSuccess) return e;
+  // Parts of at most kDirectSpan FFTs, the length over which sums were rounded to FP32 uncompensated before; more (a
+  // power of two) while SMs would stay idle and a part keeps a whole drain period.  Parts are whole stages, so the last
+  // one may be short, or empty: its CTA then adds zeros.
+  const int ngrp = nchan / p.CS;
+  p.kparts = 1;
+  while (p.kparts < 8 && (nfft > p.kparts * kDirectSpan || (ngrp * p.kparts < nsm && nfft >= 256 * p.kparts)))
+    p.kparts *= 2;
+  p.kspan = ((nfft + p.kparts - 1) / p.kparts + KC - 1) / KC * KC;
+  CUtensorMap tmap;
+  e = raw_tensor_map(&tmap, ants, 8, nchan, p.rbx, nfft, (size_t)fftwidth * 8, p.rkc, p.nstream,
+                     (size_t)nfft * fftwidth * 8, p.nstream, CW * 8);
+  if (e != cudaSuccess) return e;
+  return f16 ? launch_split<2>(p.R, p, tmap, kSplitSmem, s) : launch_split<3>(p.R, p, tmap, kSplitSmem, s);
+}
+
 cudaError_t launch_xstage_tensor(const void *chan, int chan_type, int nant, int nchan, int T, int nt, int autos,
                                  float2 *vsum, float2 *vcomp, cudaStream_t s, int split_e, int kparts_max,
                                  size_t plane, bool first) {
@@ -1505,6 +1653,7 @@ cudaError_t launch_xstage_tensor(const void *chan, int chan_type, int nant, int 
   p.kspan = nt;
   p.plane = plane;
   p.first = first;
+  p.out = nullptr;
   // FP32 data: FP16 hi/lo split of values scaled by 2^-split_e when split_e >= 0, else TF32 split
   const bool h16 = chan_type == CHAN_F32 && split_e >= 0;
   p.split_sc = h16 ? ldexpf(1.0f, -split_e) : 1.0f;
@@ -1553,7 +1702,10 @@ cudaError_t launch_xstage_tensor(const void *chan, int chan_type, int nant, int 
       kc % (chan_type == CHAN_F8 ? 16 : 8))
     return cudaErrorInvalidValue;
   CUtensorMap tmap;
-  e = raw_tensor_map(&tmap, chan, esz, p.nstream, nt, T, nchan, p.rbx, kc);
+  const size_t row = (size_t)CW * esz;
+  // the channelised block [ctile][T][n][16], the FFT extent cut at nt
+  e = raw_tensor_map(&tmap, chan, esz, nchan, p.rbx, p.nstream, row, p.nstream, nt, row * p.nstream, kc,
+                     row * p.nstream * T);
   if (e != cudaSuccess) return e;
   const size_t smem = (size_t)tc::STAGES * 65536 + (size_t)tc::RSTAGES * tc::RAW_BYTES + 1024;
   static_assert(tc::Cfg<true>::STAGE_BYTES == 65536 && tc::Cfg<false>::STAGE_BYTES == 65536, "stage size");
@@ -1562,23 +1714,7 @@ cudaError_t launch_xstage_tensor(const void *chan, int chan_type, int nant, int 
     const size_t nbl = (size_t)nant * (nant - 1) / 2 + (autos ? nant : 0);
     if (nbl * 4 * p.CS * sizeof(float2) > (size_t)tc::STAGES * tc::Cfg<true>::STAGE_BYTES || (p.CS & (p.CS - 1)))
       return cudaErrorInvalidValue;
-    auto launch = [&](auto kern) -> cudaError_t {
-      cudaError_t e2 = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e2 != cudaSuccess) return e2;
-      kern<<<nchan / p.CS, tc::NTHREADS_SPLIT, smem, s>>>(p, tmap);
-      return cudaSuccess;
-    };
-    switch (R * 2 + (h16 ? 1 : 0)) {
-      case 32: e = launch(tc::xstage_tc_split_kernel<16, false>); break;
-      case 33: e = launch(tc::xstage_tc_split_kernel<16, true>); break;
-      case 64: e = launch(tc::xstage_tc_split_kernel<32, false>); break;
-      case 65: e = launch(tc::xstage_tc_split_kernel<32, true>); break;
-      case 128: e = launch(tc::xstage_tc_split_kernel<64, false>); break;
-      case 129: e = launch(tc::xstage_tc_split_kernel<64, true>); break;
-      case 256: e = launch(tc::xstage_tc_split_kernel<128, false>); break;
-      case 257: e = launch(tc::xstage_tc_split_kernel<128, true>); break;
-      default: return cudaErrorInvalidValue;
-    }
+    e = h16 ? launch_split<1>(R, p, tmap, smem, s) : launch_split<0>(R, p, tmap, smem, s);
     if (e != cudaSuccess) return e;
   } else {
     // one CTA per SM (its shared memory): when the channel groups leave SMs idle (fewer groups

@@ -360,7 +360,10 @@ gxc_status gxc_dada_close(gxc_dada_reader *r);
  * summed over the nfft spectra and divided by nfft as CCAH3 does
  * (gcorr/src/gxkernel.cu:574-581).  precision: GXC_PRECISION_FP32 or _FP16
  * (values cast to FP16 unscaled); x_engine: GXC_XENGINE_* (as for gxc_config).  Synchronous on
- * `stream`; allocates its scratch with cudaMalloc. */
+ * `stream`; host buffers are staged in device memory, and shapes that the tensor-core
+ * X-stage cannot read in place (more than 32 antennas or 8192 FFTs, FP8, an odd
+ * fftwidth, data not 16-byte aligned, the CUDA-core engine) take scratch, both from
+ * cudaMalloc. */
 gxc_status gxc_xcorr(const float *ants, int nant, int nfft, int nchan, int fftwidth, int precision, int x_engine,
                      int autos, float *accum, void *stream);
 
