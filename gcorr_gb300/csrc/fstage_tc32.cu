@@ -8,10 +8,12 @@
 // D1 (rows (window, k1), 64 of them; columns n2) = A1 B1^T per polarisation, real and imaginary part, K = (window,
 // n1).  The fringe rotator of sample n is exp(-2 pi i (c0 + c1 n)): its n1 part is folded into A1 (rows k1 of
 // window w: W_N1^(n1 k1) e^(-2 pi i 128 n1 c1), block-diagonal over the 64 / N1 windows of a group), its n2 part into
-// the twiddles of step 2.  A1 is split into FP16 hi and lo halves (22 significand bits); the levels 1 and 3.3359 are
-// FP16 hi and lo values exactly (3.3359f = 3.3359375 - 628 x 2^-24), so D1 = A_lo B_hi + A_hi B_lo + A_hi B_hi
-// (in this order: the small terms first, so that tensor memory's rounding toward zero acts on the sum only four
-// times) drops nothing above 2^-22.
+// the twiddles of step 2.  A1 is split into FP16 hi and lo halves (22 significand bits).  B1 holds the levels times
+// 1039: 1039 and 3466 are FP16 values, and 3466 / 1039 is 3.3359 to 2.9e-8 (3.3359f is off by 2.0e-8, half a unit of its
+// last bit being 3.6e-8).  D1 = A_lo B + A_hi B, in this order: the small terms first, so that tensor memory's rounding
+// toward zero acts on the sum only four times.  An exact hi and lo pair of levels (3.3359375 - 628 x 2^-24) took half as
+// many MMAs again and twice the decode's stores, 25.1 against 24.2 ms (16 antennas, 62500 FFTs), for the same error:
+// power spectra 2.3e-7 rms from FP64 at 8192 points, 3.1e-7 at 4096, 4.1e-7 at 2048.
 // Step 2, the 128-point DFTs over n2, runs on the CUDA cores in FP32: a thread owns one row, so the transform needs no
 // exchange between threads.  Radix 8 over j (n2 = i + 16 j), back to tensor memory, radix 16 over i.  With
 // theta = k1 / N + c1 both passes take their twiddles as powers of e^(-2 pi i theta) (the DFT at a shifted
@@ -24,9 +26,9 @@
 //
 // What bounds it (16 antennas, 8192 points, FP32, 2048 FFTs, ncu): 42 instructions per complex sample (53 for the packed
 // register FFT) at 73 % issue active, FMA pipe 58 % (decode, twiddles and butterflies), tensor pipe 41 %, DRAM 32 %; a
-// team waits 3,600 clocks per group for its slot's 48 MMAs (M = 64, 64 clocks each).  F-stage of the 16-antenna,
-// nchan-4096 workload (62500 FFTs), FP32: 25.1 ms; 40.8 ms for the register FFT (fstage_pair_kernel); 6 antennas, nchan
-// 1024, 15625 FFTs: 0.60 against 0.98 ms.  On the way: eight transform warps on one group at a time, A1 rebuilt for every
+// team waited 3,600 clocks per group for its slot's MMAs (M = 64, 64 clocks each) when there were 48 of them; now 32.  F-stage of the 16-antenna,
+// nchan-4096 workload (62500 FFTs), FP32: 24.2 ms; 40.8 ms for the register FFT (fstage_pair_kernel); 6 antennas, nchan
+// 1024, 15625 FFTs: 0.57 against 0.98 ms.  On the way: eight transform warps on one group at a time, A1 rebuilt for every
 // window, 29.9 ms; the slope check with two decode teams 33.1 ms (the B1 of a slot then waits for its own MMAs); teams on
 // alternate groups 32.4; the MMA descriptors as two words 29.0; the one-word-past loads issued as one instead of a chain
 // 27.1; 16 transform warps, radix 8 x 16 instead of 16 x 8 (half the registers) 26.2.
@@ -64,7 +66,7 @@ struct Plan {
   // fst[w][k2] = e^(2 pi i N1 k2 cf) * scale
   static constexpr int T_FSUB = 0, T_E = 64, T_FST = 64 + 8 * NW, TAB = T_FST + NK2 * NW;
   // shared-memory image (byte offsets from a 1024-aligned base)
-  static constexpr int SLOT = 4 * HB + 4 * KB;  // A1: [re, im][hi, lo]; B1: [pol][hi, lo]
+  static constexpr int SLOT = 4 * HB + 2 * KB;  // A1: [re, im][hi, lo]; B1: [pol]
   static constexpr int OFF_STAGE = NS * SLOT;             // per slot: the packed windows, realigned
   static constexpr int OFF_TAB = OFF_STAGE + NS * 4096;
   static constexpr int OFF_TST = OFF_TAB + NR * TAB * 8;  // per slot: tstep[(w, n1)] of its A1
@@ -88,9 +90,13 @@ struct Params {
 
 __device__ int g_f32tc_err;
 
-// Tensor memory rounds its FP32 sums toward zero, which leaves the spectra low; A1's lo half carries the inverse.
-// Measured over 1024 to 8192 points: without it power spectra come out 1.9e-7 low on average, with it within 0.3e-7.
-constexpr float kRz = 9.5e-8f;
+// Tensor memory rounds its FP32 sums toward zero, which leaves the spectra low, and 3466 / 1039 is 4.9e-8 below 3.3359f;
+// A1's lo half carries the inverse.  Measured: with 9.5e-8 power spectra come out 1.5e-7 low on average, with this
+// value within 0.2e-7 (2048 to 8192 points).
+constexpr float kRz = 1.7e-7f;
+
+// A1 carries 2^10 / 1039 (FP16 holds it well), the frac-delay table 2^-10.
+constexpr float kScale = 1024.0f / 1039.0f;
 
 // Tensor-memory column (= row of B1) of sample n2 = i + 16 j (i < 16, j < 8): 16 pr + 2 (j xor pr / 2) + (i mod 2) with
 // pr = i / 2.  Samples i, i + 1 are adjacent columns, the lanes of packed FP32 pairs, and the eight j of a pair are 16
@@ -101,17 +107,13 @@ __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
   return *reinterpret_cast<const uint32_t *>(&h);
 }
 
-// FP16 hi and lo parts of the levels of four 2-bit codes, one per byte of `codes` (the other bits are ignored): hi of
-// {-HiMag, -1, 1, HiMag} and HiMag - 3.3359375 = -628 x 2^-24 (a subnormal), sign included.  The low bytes of the four
-// values are one word, the high bytes another: code c picks bytes c and 4 + c.
-__device__ __forceinline__ void level_quad(uint32_t codes, uint32_t (&hi)[2], uint32_t (&lo)[2]) {
-  constexpr uint32_t kHiL = 0xAC0000ACu, kHiH = 0x423CBCC2u;  // 0xC2AC, 0xBC00, 0x3C00, 0x42AC
-  constexpr uint32_t kLoL = 0x74000074u, kLoH = 0x82000002u;  // 0x0274, 0, 0, 0x8274
+// Scaled FP16 levels of four 2-bit codes, one per byte of `codes` (the other bits are ignored): {-3466, -1039, 1039, 3466}.
+// Their low bytes are one word, their high bytes another: code c picks bytes c and 4 + c.
+__device__ __forceinline__ void level_quad(uint32_t codes, uint32_t (&v)[2]) {
+  constexpr uint32_t kL = 0xC50F0FC5u, kH = 0x6A64E4EAu;  // 0xEAC5, 0xE40F, 0x640F, 0x6AC5
   const uint32_t sel = (codes & 0x03030303u) * 0x11u + 0x40404040u;
-  hi[0] = tc::prmt(kHiL, kHiH, sel);
-  lo[0] = tc::prmt(kLoL, kLoH, sel);
-  hi[1] = tc::prmt(kHiL, kHiH, sel >> 16);
-  lo[1] = tc::prmt(kLoL, kLoH, sel >> 16);
+  v[0] = tc::prmt(kL, kH, sel);
+  v[1] = tc::prmt(kL, kH, sel >> 16);
 }
 
 // Group of NW consecutive FFTs of one antenna; a CTA takes a contiguous run of groups, FFTs fastest, so that the
@@ -458,7 +460,7 @@ __global__ void __launch_bounds__(NT, 1) fstage_tc32_kernel(Params p) {
         } else {
           const int y = x - P::T_FST;
           arg = 2.0f * ((float)(N1 * (y % P::NK2)) * gg[y / P::NK2].cf);
-          sc = p.out_scale;  // a power of two: exact
+          sc = p.out_scale * 0x1p-10f;  // powers of two: exact
         }
         float sn, cs;
         sincospif(arg, &sn, &cs);
@@ -472,12 +474,12 @@ __global__ void __launch_bounds__(NT, 1) fstage_tc32_kernel(Params p) {
       if (rebuild) {
         if (s) a1_slope[1] = slope;
         else a1_slope[0] = slope;
-        if (gt < 64) {  // row gt of tstep: (w, n1)
+        if (gt < 64) {  // row gt of tstep: (w, n1), with the levels' scale
           const float m = (float)(gt % N1) * smul, ph = m * slope.x;
           const float lo = -6.283185307f * fmaf(m, slope.y, fmaf(m, slope.x, -ph));
           float sn, cs;
           sincospif(-2.0f * ph, &sn, &cs);
-          tst[gt] = make_float2(fmaf(-sn, lo, cs), fmaf(cs, lo, sn));
+          tst[gt] = make_float2(fmaf(-sn, lo, cs) * kScale, fmaf(cs, lo, sn) * kScale);
         }
       }
       uint32_t vm = 0;  // valid windows
@@ -518,21 +520,20 @@ __global__ void __launch_bounds__(NT, 1) fstage_tc32_kernel(Params p) {
 #pragma unroll
           for (int pol = 0; pol < 2; pol++) {
             const int sh = 4 * (r & 1) + 2 * pol;
-            uint32_t h0[2], l0[2], h1[2], l1[2];
-            level_quad(t[r0 >> 1][0] >> sh, h0, l0);
-            level_quad(t[r0 >> 1][1] >> sh, h1, l1);
-            *reinterpret_cast<uint4 *>(dst + 2 * pol * KB) = make_uint4(h0[0], h0[1], h1[0], h1[1]);
-            *reinterpret_cast<uint4 *>(dst + (2 * pol + 1) * KB) = make_uint4(l0[0], l0[1], l1[0], l1[1]);
+            uint32_t h0[2], h1[2];
+            level_quad(t[r0 >> 1][0] >> sh, h0);
+            level_quad(t[r0 >> 1][1] >> sh, h1);
+            *reinterpret_cast<uint4 *>(dst + pol * KB) = make_uint4(h0[0], h0[1], h1[0], h1[1]);
             if constexpr (DBG) {
               const int w = 8 * o / N1, tl = cur.tg * NW + w;
               if ((vm >> w) & 1u) {
                 float2 *pr = p.probe + (((size_t)cur.ant * 2 + pol) * job.nfft + (p.t0 + tl)) * N + 4 * lane + r;
 #pragma unroll
                 for (int j = 0; j < 8; j++) {
-                  const uint32_t hb = j < 4 ? h0[j >> 1] : h1[(j - 4) >> 1], lb = j < 4 ? l0[j >> 1] : l1[(j - 4) >> 1];
-                  const __half2 h2 = *reinterpret_cast<const __half2 *>(&hb), l2 = *reinterpret_cast<const __half2 *>(&lb);
-                  const float2 hf = __half22float2(h2), lf = __half22float2(l2);
-                  pr[128 * ((8 * o) % N1 + j)] = make_float2((j & 1) ? hf.y + lf.y : hf.x + lf.x, 0.f);
+                  const uint32_t hb = j < 4 ? h0[j >> 1] : h1[(j - 4) >> 1];
+                  const float2 hf = __half22float2(*reinterpret_cast<const __half2 *>(&hb));
+                  const float v = (j & 1) ? hf.y : hf.x;
+                  pr[128 * ((8 * o) % N1 + j)] = make_float2(copysignf(fabsf(v) > 2000.0f ? 3.3359f : 1.0f, v), 0.f);
                 }
               }
             }
@@ -586,12 +587,11 @@ __global__ void __launch_bounds__(NT, 1) fstage_tc32_kernel(Params p) {
 #pragma unroll
           for (int pol = 0; pol < 2; pol++) {
             const uint32_t d = tmem0 + 256u * s + 128 * part + ((uint32_t)(16 * pol) << 16);
-            const uint32_t ah = a1 + 2 * part * HB / 16, bh = b1 + 2 * pol * KB / 16;
+            const uint32_t ah = a1 + 2 * part * HB / 16, bh = b1 + pol * KB / 16;
             mma_f16_lo<false>(d, ah + HB / 16, bh, IDESC_M64);
 #pragma unroll
-            for (int x = 1; x < 12; x++)  // A_lo B_hi, A_hi B_lo, A_hi B_hi, four K steps each
-              mma_f16_lo<true>(d, ah + (x < 4 ? HB / 16 : 0) + 2 * (x & 3), bh + (x >= 4 && x < 8 ? KB / 16 : 0) + 2 * (x & 3),
-                               IDESC_M64);
+            for (int x = 1; x < 8; x++)  // A_lo B, A_hi B, four K steps each
+              mma_f16_lo<true>(d, ah + (x < 4 ? HB / 16 : 0) + 2 * (x & 3), bh + 2 * (x & 3), IDESC_M64);
           }
         mma_commit(smem_u32(&ab_free[s]));
         mma_commit(smem_u32(&d_full[s]));
