@@ -390,7 +390,7 @@ gxc_status gxc_create(const gxc_config *cfg, gxc_handle **out) {
   h->tc_fstage = cfg->fft_engine != GXC_FFT_CUDA_CORE && fstage_tc_supported(j, h->chan_type);
   if (e == cudaSuccess && h->tc_fstage) e = make_fstage_tc_tables(&h->d_tc_tables);
   // otherwise the FP32-accurate F-stage: its first step on tensor cores where that is faster, else the register FFT
-  h->tc32_fstage = !h->tc_fstage && fstage_tc32_worth(j, h->T);
+  h->tc32_fstage = !h->tc_fstage && fstage_tc32_worth(j, h->T, h->chan_type);
   if (h->chan_type == CHAN_F8 && cfg->fp8_scaling == GXC_FP8_SCALE_CHANNEL) {
     // calibration block: up to 64 FFTs, at most 256 MB of FP32 channelised data (at least 4 FFTs)
     const size_t per_fft32 = (size_t)cfg->nchan * 2 * nant * sizeof(float2);

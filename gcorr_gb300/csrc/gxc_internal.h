@@ -91,10 +91,10 @@ cudaError_t launch_fstage_tc(const Job &job, const void *tables, int t0, int nt,
                              float2 *probe = nullptr);
 cudaError_t fstage_tc_take_error(int *flag);
 
-// fstage_tc32.cu: the F-stage in FP32 accuracy with its first step on tensor cores (2048- to 8192-point windows, 2-bit
-// real), every channelised type.  T: the handle's FFT block.  probe as for launch_fstage_tc.
-int fstage_tc32_supported(const Job &job, int T);
-int fstage_tc32_worth(const Job &job, int T);  // supported, and faster than the register FFT at this size
+// fstage_tc32.cu: the F-stage in FP32 accuracy with its first step on tensor cores (2-bit real windows; 2048 to 8192 points
+// with every channelised type, 16384 and 32768 points with FP32).  T: the handle's FFT block.  probe as for launch_fstage_tc.
+int fstage_tc32_supported(const Job &job, int T, int chan_type);
+int fstage_tc32_worth(const Job &job, int T, int chan_type);  // supported, and faster than the register FFT at this size
 cudaError_t launch_fstage_tc32(const Job &job, int t0, int nt, int T, void *chan, int chan_type, float out_scale,
                                cudaStream_t s, const float *cscale = nullptr, float2 *probe = nullptr);
 cudaError_t fstage_tc32_take_error(int *flag);

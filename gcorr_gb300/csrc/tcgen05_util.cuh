@@ -272,6 +272,8 @@ constexpr uint32_t IDESC = (1u << 4) | (0u << 7) | (0u << 10) | ((128u >> 3) << 
 // M = 64, N = 128, A = B = F16: rows 16 i .. 16 i + 15 of D are the lanes 32 i .. 32 i + 15 of its tensor-memory
 // address, so two of them share columns at lanes 0 and 16.
 constexpr uint32_t IDESC_M64 = (1u << 4) | (0u << 7) | (0u << 10) | ((128u >> 3) << 17) | ((64u >> 4) << 24);
+// M = 128, N = 256, A = B = F16
+constexpr uint32_t IDESC_N256 = (1u << 4) | (0u << 7) | (0u << 10) | ((256u >> 3) << 17) | ((128u >> 4) << 24);
 constexpr uint32_t IDESC_TF32 = (1u << 4) | (2u << 7) | (2u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
 
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {

@@ -969,7 +969,6 @@ __global__ void __launch_bounds__(NTHREADS_SPLIT, 1) xstage_tc_split_kernel(Para
 // 384 of the 512 TMEM columns; one 32 KiB stage per 64 FFTs (4 stages).
 constexpr int BIG_STAGES = 4;
 constexpr int BIG_STAGE_BYTES = 256 * 128;
-constexpr uint32_t IDESC_N256 = (1u << 4) | ((256u >> 3) << 17) | ((128u >> 4) << 24);
 
 template <bool F8>
 __global__ void __launch_bounds__(NTHREADS, 1) xstage_tc_big_kernel(Params p) {
