@@ -66,7 +66,7 @@ struct Cfg {
 struct Params {
   const void *chan;     // [ctile][T][n][16] half2 (FP16 path) or float2 (SPLIT path)
   int nant, nstream, nchan, T, nt, autos;
-  int R, g, CS;         // rows per channel block, channels per MMA group, channels per CTA
+  int R, g, CS, ng;     // rows per channel block, channels per MMA group, channels per CTA = ng groups of g
   float2 *vsum, *vcomp;
   int *err;
   // TMA raw tiles (small-N kernels): box = rbx channels x nstream x rkc FFTs, rnbox boxes
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(NTHREADS_TC, 1) xstage_tc_kernel(Params p, con
   auto zero_padding = [&](int t0, int nthr) {
     if (2 * n >= p.R) return;
     const int pad = p.R - 2 * n;
-    const int per_stage = NG * p.g * pad * 8;  // 16-byte words
+    const int per_stage = p.ng * p.g * pad * 8;  // 16-byte words
     for (int i = t0; i < STAGES * per_stage; i += nthr) {
       const int st = i / per_stage, r0 = i - st * per_stage;
       const int w = r0 & 7, rr = r0 >> 3;
@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(NTHREADS_TC, 1) xstage_tc_kernel(Params p, con
           const int col0 = gi0 * p.R;
           const int clen = p.R > 32 ? p.R : 32;
           const int j = s1 >> 1, l = s1 & 1;
-          for (int G = warp >> 2; G < NG; G += 2) {
+          for (int G = warp >> 2; G < p.ng; G += 2) {
             const int cl = G * p.g + my_gi;  // channel within the CTA's CS
             for (int pc = 0; pc < clen; pc += 16) {
               __syncwarp();  // tcgen05.ld is warp-collective: reconverge after the divergent skip below
@@ -499,6 +499,7 @@ __global__ void __launch_bounds__(NTHREADS_TC, 1) xstage_tc_kernel(Params p, con
         const uint32_t sa = sbase + st * STAGE_BYTES;
 #pragma unroll
         for (int G = 0; G < NG; G++) {
+          if (G >= p.ng) break;
 #pragma unroll
           for (int kk = 0; kk < KC / KSTEP; kk++) {
             const uint32_t acc = (k > k0 || kk > 0) ? 1u : 0u;
@@ -588,7 +589,7 @@ __global__ void __launch_bounds__(NTHREADS_SPLIT, 1) xstage_tc_split_kernel(Para
 
   if (2 * n < R) {  // zero the padding rows of both tiles (hi, lo) of every group of every stage
     const int pad = R - 2 * n;
-    const int per_stage = NG * GCH * pad * 8 * 2;
+    const int per_stage = p.ng * GCH * pad * 8 * 2;
     for (int i = tid; i < STAGES * per_stage; i += NTHREADS_SPLIT) {
       const int st = i / per_stage, r0 = i - st * per_stage;
       const int w = r0 & 7, rr = (r0 >> 3) >> 1, tile = (r0 >> 3) & 1;
@@ -797,6 +798,7 @@ __global__ void __launch_bounds__(NTHREADS_SPLIT, 1) xstage_tc_split_kernel(Para
         const uint32_t sa = sbase + st * STAGE_BYTES;
 #pragma unroll
         for (int G = 0; G < NG; G++) {
+          if (G >= p.ng) break;
           const uint32_t d = tmem + b * SET_COLS + G * 128;
 #pragma unroll
           for (int kk = 0; kk < KC / KSTEP; kk++) {
@@ -842,6 +844,7 @@ __global__ void __launch_bounds__(NTHREADS_SPLIT, 1) xstage_tc_split_kernel(Para
       tc_fence_after();
 #pragma unroll
       for (int G = 0; G < NG; G++) {
+        if (G >= p.ng) break;
 #pragma unroll
         for (int pw = 0; pw < WP; pw++) {
           const int col = gi0 * R + 16 * pw;
@@ -888,6 +891,7 @@ __global__ void __launch_bounds__(NTHREADS_SPLIT, 1) xstage_tc_split_kernel(Para
       if (ok && s1 < n) {
 #pragma unroll
         for (int G = 0; G < NG; G++) {
+          if (G >= p.ng) break;
           const int cl = G * GCH + my_gi;  // channel within the CTA's CS
 #pragma unroll
           for (int a = 0; a < PP; a++) {
@@ -1592,6 +1596,7 @@ cudaError_t launch_xstage_direct(const void *ants, int chan_type, int nant, int 
   while (p.R < 2 * p.nstream) p.R <<= 1;
   p.g = 128 / p.R;
   p.CS = xstage_tensor_channels_per_cta(nant, CHAN_F32);
+  p.ng = p.CS / p.g;
   p.split_sc = p.split_unsc = 1.0f;
   p.out = out;
   const bool f16 = chan_type == CHAN_F16;
@@ -1681,10 +1686,37 @@ cudaError_t launch_xstage_tensor(const void *chan, int chan_type, int nant, int 
     kern<<<nchan, tc::NTHREADS, bsmem, s>>>(p);
     return cudaGetLastError();
   }
-  // small-N kernels: raw TMA tiles of rbx channels (at least 16 bytes: FP8 with 4 channels per
-  // CTA loads 8, of which the CTA uses its 4) x all streams x rkc FFTs, one box per channel tile
+  // small-N kernels.  The FP16 / FP8 kernel splits the block's FFTs across two CTAs per channel group, or runs persistent
+  // (xstage_seg); both kernels then take fewer MMA groups per CTA while that still fits the SMs in one wave, which
+  // leaves every sum as it was: 7 antennas, 512 channels, 32003 FFTs, FP16 (64 CTAs, now 128) 0.32 -> 0.21 ms.
+  int dev = 0, nsm = 0;
+  e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
   const int esz = (int)chan_elem_bytes(chan_type);
   const int KC = chan_type == CHAN_F32 ? (h16 ? 64 : tc::Cfg<true>::KC) : chan_type == CHAN_F8 ? 128 : tc::Cfg<false>::KC;
+  const int ngrp = nchan / p.CS;
+  if (chan_type != CHAN_F32) {
+    // one CTA per SM (its shared memory): when the channel groups leave SMs idle (fewer groups
+    // than SMs), split the block's FFTs in two halves, each into its own accumulator plane (with
+    // nt >= 4 KC both halves hold more than KC FFTs, so no CTA accumulates nothing).  Measured:
+    // 6 antennas (64 groups) FP16 0.49 -> 0.30 ms; with 512 groups (3.4 waves) the split was
+    // slower (9.0 -> 10.3 ms), its halved CTAs paying their pipeline fill and drain twice.
+    if (plane > 0 && splits_block(ngrp, nsm, nt, KC, kparts_max)) {
+      p.kparts = 2;
+      p.kspan = (nt / 2 + KC - 1) / KC * KC;
+    } else if (kparts_max == 2 && plane > 0 && ngrp >= nsm) {
+      // at least as many groups as SMs: one CTA per SM, each an equal share of all (group, K
+      // chunk) units, so no SM idles in a last partial wave (512 groups are 3.37 waves)
+      p.persist = 1;
+    }
+  }
+  const int cs_min = chan_type == CHAN_F32 ? 2 : 4;  // the producers take channels in pairs, in fours
+  while (!p.persist && p.CS > p.g && p.CS > cs_min && 2 * (nchan / p.CS) * p.kparts <= nsm) p.CS /= 2;
+  p.ng = p.CS / p.g;
+  p.ngrp = nchan / p.CS;
+  // raw TMA tiles of rbx channels (at least 16 bytes: FP8 with 4 channels per
+  // CTA loads 8, of which the CTA uses its 4) x all streams x rkc FFTs, one box per channel tile
   p.rnbox = p.CS > CW ? p.CS / CW : 1;
   p.rbx = p.CS > CW ? CW : (p.CS * esz >= 16 ? p.CS : 16 / esz);
   if (p.rbx * esz < 16 || p.rbx > CW || (p.CS > CW && p.CS % CW)) return cudaErrorInvalidValue;
@@ -1716,35 +1748,15 @@ cudaError_t launch_xstage_tensor(const void *chan, int chan_type, int nant, int 
     e = h16 ? launch_split<1>(R, p, tmap, smem, s) : launch_split<0>(R, p, tmap, smem, s);
     if (e != cudaSuccess) return e;
   } else {
-    // one CTA per SM (its shared memory): when the channel groups leave SMs idle (fewer groups
-    // than SMs), split the block's FFTs in two halves, each into its own accumulator plane (with
-    // nt >= 4 KC both halves hold more than KC FFTs, so no CTA accumulates nothing).  Measured:
-    // 6 antennas (64 groups) FP16 0.49 -> 0.30 ms; with 512 groups (3.4 waves) the split was
-    // slower (9.0 -> 10.3 ms), its halved CTAs paying their pipeline fill and drain twice.
-    const int ngrp = nchan / p.CS;
     // each segment epilogue stages [baseline x product][CS] visibilities in the operand ring
     const size_t nbl = (size_t)nant * (nant - 1) / 2 + (autos ? nant : 0);
     if (nbl * 4 * p.CS * sizeof(float2) > (size_t)tc::STAGES * tc::Cfg<false>::STAGE_BYTES ||
         (p.CS & (p.CS - 1)))
       return cudaErrorInvalidValue;
-    int dev = 0, nsm = 0;
-    e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return e;
-    p.ngrp = ngrp;
-    p.persist = 0;
-    if (plane > 0 && splits_block(ngrp, nsm, nt, KC, kparts_max)) {
-      p.kparts = 2;
-      p.kspan = (nt / 2 + KC - 1) / KC * KC;
-    } else if (kparts_max == 2 && plane > 0 && ngrp >= nsm) {
-      // at least as many groups as SMs: one CTA per SM, each an equal share of all (group, K
-      // chunk) units, so no SM idles in a last partial wave (512 groups are 3.37 waves)
-      p.persist = 1;
-    }
     auto kern = chan_type == CHAN_F8 ? tc::xstage_tc_kernel<true> : tc::xstage_tc_kernel<false>;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    kern<<<p.persist ? nsm : ngrp * p.kparts, tc::NTHREADS_TC, smem, s>>>(p, tmap);
+    kern<<<p.persist ? nsm : p.ngrp * p.kparts, tc::NTHREADS_TC, smem, s>>>(p, tmap);
   }
   return cudaGetLastError();
 }
