@@ -393,6 +393,15 @@ __global__ void __launch_bounds__(NT, 1) fstage_tc_kernel(Params p) {
       if (!mbar_wait_warp(smem_u32(&tab_full[ri]), rp, p.err)) break;
       if (ring_valid[ri]) {
         const int s = c % NS;
+        // FP8: the scales of eight channels, loaded one step ahead (before the wait for the first ones).  Loaded where they
+        // were used they held this role up: 62500 FFTs of 16 antennas 17.4 ms, now 16.7 (FP16 without scales 14.8)
+        constexpr bool SCALED = std::is_same<OutT, __nv_fp8x2_e4m3>::value;
+        float scn[8];
+        auto load_scales = [&](int jj) {
+#pragma unroll
+          for (int e = 0; e < 8; e++) scn[e] = chan_scale<OutT>(csc, 64 * (8 * jj + e), 1.0f);
+        };
+        if constexpr (SCALED) load_scales(0);
         if (!mbar_wait_warp(smem_u32(&d3_full[s]), (c / NS) & 1, p.err)) break;
         tc_fence_after();
         const uint32_t trow = tmem0 + 256u * s + ((uint32_t)(32 * q) << 16) + 64u * h;
@@ -402,6 +411,12 @@ __global__ void __launch_bounds__(NT, 1) fstage_tc_kernel(Params p) {
         for (int jj = 0; jj < 4; jj++) {
           float v[16];
           tmem_ld16_async(trow + 16 * jj, v);
+          float sc[8];
+#pragma unroll
+          for (int e = 0; e < 8; e++) sc[e] = SCALED ? scn[e] : 1.0f;
+          if constexpr (SCALED) {
+            if (jj < 3) load_scales(jj + 1);
+          }
           tmem_wait_ld16(v);
           if (jj == 3) {  // D3 has been read: step 1 of the slot's next window may overwrite it
             tc_fence_before();
@@ -416,9 +431,9 @@ __global__ void __launch_bounds__(NT, 1) fstage_tc_kernel(Params p) {
             const float2 zr = csub(pmul(VR, FR), pmul(VI, FI)), zi = pfma(VR, FI, pmul(VI, FR));
             const uint32_t k2 = 8 * jj + 2 * e;
             *reinterpret_cast<OutT *>(o + (uint64_t)k2 * step) =
-                to_out<OutT>(make_float2(zr.x, zi.x), chan_scale<OutT>(csc, 64 * k2, 1.0f));
+                to_out<OutT>(make_float2(zr.x, zi.x), sc[2 * e]);
             *reinterpret_cast<OutT *>(o + (uint64_t)(k2 + 1) * step) =
-                to_out<OutT>(make_float2(zr.y, zi.y), chan_scale<OutT>(csc, 64 * (k2 + 1), 1.0f));
+                to_out<OutT>(make_float2(zr.y, zi.y), sc[2 * e + 1]);
           }
         }
         c++;
