@@ -56,7 +56,7 @@ __global__ void geometry_kernel(Job job, const __grid_constant__ GeomParams u, i
     const double br = b - (double)intdelay;
     double c0 = br * job.lo_hz;
     if (job.fractional_lo) c0 += (job.lo_hz - trunc(job.lo_hz)) * (double)intdelay;
-    c0 -= rint(c0);
+    c0 -= floor(c0);
     const double c1 = a * job.lo_hz * job.inv_F;  // turns per sample (F is a power of two)
     // coarse step: the reference advances its step table by `stride` samples per
     // entry (fxkernel.cpp:112) while applying it every `substride` samples;

@@ -141,13 +141,14 @@ struct FParams {
   const float2 *tw;    // W_F^m, m < F
   const float2 *twp1;  // F = 8192: pass-1 twiddles of the packed-pair kernel (make_twiddles), else null
   const float2 *twp2;  // F = 8192: pass-2 twiddles of the packed-pair kernel, else null
-  int t0, nt, T;
+  int t0, T;
   void *chan;
   float out_scale;
   int sub_shift, sub_mask;    // substride = 1 << sub_shift
   int fsub_shift, fsub_mask;  // fsub = 1 << fsub_shift
   float2 *probe;              // DBG kernels: decoded samples [nant][2][nfft][F] before rotation
   const float *cscale;        // FP8 output: per-channel scale [nchan] (replaces out_scale), or null
+  int nt;                     // FFTs of the launch
 };
 
 // Output scale of channel c: FP8 output with per-channel scales uses cscale[c] (the caller then

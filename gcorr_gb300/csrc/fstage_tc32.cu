@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(Plan<L>::NT, 1) fstage_tc32_kernel(Params p) {
         } else if (x < P::T_FST) {
           const Geom &gw = gg[(unsigned)(x - P::T_E) / P::ES];
           const int sft = (x - P::T_E) & (P::ES - 1);
-          arg = -2.0f * (sft < NP ? (float)(1 << sft) * gw.c1 : gw.c0);
+          arg = -2.0f * (sft < NP ? (float)(1 << sft) * gw.c1 : gw.c0 - rintf(gw.c0));  // (the phase mod 1: exact)
           lo = -6.283185307f * (sft < NP ? (float)(1 << sft) * gw.c1_lo : gw.c0_lo);
           if (sft == NP) sc = gw.valid ? 1.0f : 0.0f;
         } else {

@@ -27,6 +27,7 @@ struct gxc_handle {
   int chan_type = CHAN_F32;
   int xeng = GXC_XENGINE_CUDA_CORE;
   bool tc_fstage = false;  // tensor-core F-stage (fstage_tc.cu)
+  bool tc_cross = false;   // ... in the form for handles without autocorrelations (fstage_tc_cross.cu)
   bool tc32_fstage = false;  // FP32-accurate F-stage with its first step on tensor cores (fstage_tc32.cu)
   void *d_tc_tables = nullptr;
   float out_scale = 1.f;   // applied to channelised values before the cast
@@ -388,9 +389,15 @@ gxc_status gxc_create(const gxc_config *cfg, gxc_handle **out) {
   // FP8 channelised data): 15.4 ms against 40.1 ms for the CUDA-core FFT per second of the
   // 16-antenna, 512 Ms/s workload at FP16
   h->tc_fstage = cfg->fft_engine != GXC_FFT_CUDA_CORE && fstage_tc_supported(j, h->chan_type);
-  if (e == cudaSuccess && h->tc_fstage) e = make_fstage_tc_tables(&h->d_tc_tables);
+  // Results without autocorrelations are mostly noise, whose low bits are those of the FP16 or FP8 roundings of the spectra;
+  // they keep the kernels whose FP32 roundings they have (2-norm of the change otherwise: FP16 at 8192 points 8.5e-5 after
+  // 2500 FFTs, at 2048 and 4096 points 1.6e-5; FP8 1e-4 to 1e-3 after 50000)
+  const bool cross_only = !cfg->autos && h->chan_type != CHAN_F32;
+  h->tc_cross = h->tc_fstage && cross_only;
+  if (e == cudaSuccess && h->tc_fstage)
+    e = h->tc_cross ? make_fstage_tc_cross_tables(&h->d_tc_tables) : make_fstage_tc_tables(&h->d_tc_tables);
   // otherwise the FP32-accurate F-stage: its first step on tensor cores where that is faster, else the register FFT
-  h->tc32_fstage = !h->tc_fstage && fstage_tc32_worth(j, h->T, h->chan_type);
+  h->tc32_fstage = !h->tc_fstage && !cross_only && fstage_tc32_worth(j, h->T, h->chan_type);
   if (h->chan_type == CHAN_F8 && cfg->fp8_scaling == GXC_FP8_SCALE_CHANNEL) {
     // calibration block: up to 64 FFTs, at most 256 MB of FP32 channelised data (at least 4 FFTs)
     const size_t per_fft32 = (size_t)cfg->nchan * 2 * nant * sizeof(float2);
@@ -766,8 +773,9 @@ extern "C++" gxc_status gxc::process_chained(gxc_handle *h, void *stream, cudaEv
     const float osc = h->d_cscale ? 1.0f : h->out_scale;
     if (timing) GXC_CUDA(h, cudaEventRecord(h->ev_stage[3 * b], s), "timing event");
     if (h->tc_fstage)
-      GXC_CUDA(h, launch_fstage_tc(h->job, h->d_tc_tables, t0, nt, h->T, h->d_chan, h->chan_type, osc, s,
-                                   h->d_cscale),
+      GXC_CUDA(h,
+               (h->tc_cross ? launch_fstage_tc_cross : launch_fstage_tc)(h->job, h->d_tc_tables, t0, nt, h->T, h->d_chan,
+                                                                         h->chan_type, osc, s, h->d_cscale, nullptr),
                "tensor-core F-stage kernel");
     else if (h->tc32_fstage)
       GXC_CUDA(h, launch_fstage_tc32(h->job, t0, nt, h->T, h->d_chan, h->chan_type, osc, s, h->d_cscale),
@@ -832,8 +840,8 @@ gxc_status gxc_probe_unpack(gxc_handle *h, float *decoded) {
     const int t0 = b * h->T;
     const int nt = (c.nfft - t0) < h->T ? (c.nfft - t0) : h->T;
     // the probe runs the handle's own F-stage kernel family
-    e = h->tc_fstage ? launch_fstage_tc(h->job, h->d_tc_tables, t0, nt, h->T, chan, h->chan_type, h->out_scale,
-                                        nullptr, nullptr, probe)
+    e = h->tc_fstage ? (h->tc_cross ? launch_fstage_tc_cross : launch_fstage_tc)(
+                           h->job, h->d_tc_tables, t0, nt, h->T, chan, h->chan_type, h->out_scale, nullptr, nullptr, probe)
         : h->tc32_fstage ? launch_fstage_tc32(h->job, t0, nt, h->T, chan, h->chan_type, h->out_scale, nullptr, nullptr,
                                               probe)
                      : launch_fstage_probe(h->job, h->d_tw, t0, nt, h->T, chan, h->chan_type, h->out_scale, probe,
@@ -860,7 +868,8 @@ gxc_status gxc_sync(gxc_handle *h) {
   }
   if (h->tc_fstage) {
     int flag = 0;
-    GXC_CUDA(h, fstage_tc_take_error(&flag), "reading the F-stage status");
+    GXC_CUDA(h, h->tc_cross ? fstage_tc_cross_take_error(&flag) : fstage_tc_take_error(&flag),
+             "reading the F-stage status");
     if (flag) return fail(h, GXC_ERR_TIMEOUT, "tensor-core F-stage: a bounded device wait expired");
   }
   if (h->tc32_fstage) {

@@ -19,7 +19,7 @@ constexpr int CW = 16;
 // constants of the F-stage are evaluated there in FP64, once per (antenna, FFT),
 // reduced mod 1 turn and rounded to FP32 (fxkernel.cpp:503-535, :600-630).
 struct Geom {
-  float c0;      // fringe phase at the first sample, turns, in [-1/2, 1/2]
+  float c0;      // fringe phase at the first sample, turns, in [0, 1]
   float c1;      // fringe phase slope, turns per sample
   float cstep;   // phase advance of one coarse rotator-table entry, turns
   float cf;      // fractional-sample correction, turns per channel
@@ -90,6 +90,13 @@ cudaError_t launch_fstage_tc(const Job &job, const void *tables, int t0, int nt,
                              float out_scale, cudaStream_t s, const float *cscale = nullptr,
                              float2 *probe = nullptr);
 cudaError_t fstage_tc_take_error(int *flag);
+
+// fstage_tc_cross.cu: the same for handles without autocorrelations (its own constant operands).
+cudaError_t make_fstage_tc_cross_tables(void **out);
+cudaError_t launch_fstage_tc_cross(const Job &job, const void *tables, int t0, int nt, int T, void *chan, int chan_type,
+                                   float out_scale, cudaStream_t s, const float *cscale = nullptr,
+                                   float2 *probe = nullptr);
+cudaError_t fstage_tc_cross_take_error(int *flag);
 
 // fstage_tc32.cu: the F-stage in FP32 accuracy with its first step on tensor cores (2-bit real windows; 2048 to 8192 points
 // with every channelised type, 16384 and 32768 points with FP32).  T: the handle's FFT block.  probe as for launch_fstage_tc.

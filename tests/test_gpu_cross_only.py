@@ -1,0 +1,29 @@
+"""FP16 and FP8 handles without autocorrelations, whose 8192-point windows take their own F-stage (fstage_tc_cross.cu):
+cross products against the FP64 oracle, from one FFT to several per SM."""
+import numpy as np
+import pytest
+
+from gcorr_gb300 import FxKernel, synth
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+TOL = {"fp16": 1e-3, "fp8": 0.12}   # the parity tests' tolerances
+
+
+@pytest.mark.parametrize("nchan", [1024, 4096])
+@pytest.mark.parametrize("precision", ["fp16", "fp8"])
+@pytest.mark.parametrize("nfft", [1, 37, 160])
+def test_crosses_vs_fp64(nchan, precision, nfft):
+    w = synth.Workload(nant=4, nchan=nchan, nfft=nfft, bw_hz=64e6, seed=nchan + nfft, offset_us=1.0, rho=0.5)
+    d = synth.generate(w)
+    fx = FxKernel(w.nant, w.nchan, w.nfft, w.nbit, w.lo_hz, w.bw_hz, precision=precision, autos=False)
+    fx.setInputData([x.cuda() for x in d["inputs"]])
+    fx.setDelays(d["poly"], d["fso"])
+    fx.process()
+    vis, counts = fx.visibilities(), fx.baseline_counts()
+    fx.close()
+    ref, rc = O.exact_process(O.config_from_workload(w, O.ROT_EXACT, False), [x.numpy() for x in d["inputs"]], d["poly"],
+                              d["fso"])
+    assert np.array_equal(counts, rc)
+    assert O.rel_rms_per_product(vis, ref).max() < TOL[precision]
