@@ -31,7 +31,7 @@
 // What bounds it (16 antennas, 2048 FFTs, ncu): 20 warp instructions per 32 samples at 56 % issue active, FMA pipe
 // 40 %, tensor pipe 45 %, shared-memory data path 40 % + 28 % for MMA operands, DRAM 28 %; a window holds its
 // tensor-memory slot for about 9,300 clocks (MMAs, 3,400 for the twiddle, 2,500 for the output), and two slots give
-// one window per 4,850.  F-stage of the 16-antenna, nchan-4096 workload, FP16, 31250 FFTs: 7.7 ms; 15.5 ms for the
+// one window per 4,850.  F-stage of the 16-antenna, nchan-4096 workload, FP16, 31250 FFTs: 7.4 ms; 15.5 ms for the
 // form before it (one 512-thread CTA that went through the phases of a window together, the intermediate in shared
 // memory written by 2-byte stores); 20.0 ms for the CUDA-core FFT.  Intermediate forms: two 256-thread groups, each
 // one window through all phases, 10.2 ms; warp roles with a block-diagonal M = 128 step 1, 8.1 ms; 16 warps that

@@ -24,9 +24,9 @@
 // A1, tables), one that issues the MMAs (and three that idle).  Two operand slots and two 256-column tensor-memory
 // slots are in flight, connected by mbarriers.
 //
-// What bounds it (16 antennas, 8192 points, FP32, 2048 FFTs, ncu): 42 instructions per complex sample (53 for the packed
-// register FFT) at 73 % issue active, FMA pipe 58 % (decode, twiddles and butterflies), tensor pipe 41 %, DRAM 32 %; a
-// team waited 3,600 clocks per group for its slot's MMAs (M = 64, 64 clocks each) when there were 48 of them; now 32.
+// What bounds it (16 antennas, 8192 points, FP32, 2048 FFTs, ncu): 40.5 instructions per sample and polarisation (53 for the
+// packed register FFT) at 73 % issue active, FMA pipe 58 % (twiddles and butterflies), tensor pipe 29 %, DRAM 35 %.  While a
+// slot had 48 MMAs (M = 64, 64 clocks each) a team waited 3,600 clocks per group for them; now they are 32.
 // F-stage of the 16-antenna, nchan-4096 workload (62500 FFTs), FP32: 24.3 ms; 40.8 ms for the register FFT (fstage_pair_kernel); 6 antennas, nchan
 // 1024, 15625 FFTs: 0.57 against 0.98 ms.  On the way: eight transform warps on one group at a time, A1 rebuilt for every
 // window, 29.9 ms; the slope check with two decode teams 33.1 ms (the B1 of a slot then waits for its own MMAs); teams on

@@ -60,10 +60,10 @@ enum { GXC_XENGINE_AUTO = 0, GXC_XENGINE_CUDA_CORE = 1, GXC_XENGINE_TENSOR = 2 }
  * operands, FP32 accumulation), for FP16 / FP8 channelised output of 8192-point
  * windows of 2-bit real data (nchan 4096); it adds four FP16 roundings inside the
  * FFT.  CUDA_CORE: the FP32-accurate FFT of every shape (FP32
- * arithmetic; for larger blocks of 2048- to 8192-point windows of 2-bit real data the
+ * arithmetic; for larger blocks of 2-bit real windows of 2048 points and more the
  * first step, whose inputs are exact, runs on tensor cores).  AUTO: TENSOR where it
- * runs, the faster of the two on GB300 (16 antennas, nchan 4096, 62500 FFTs, FP16: 15.4
- * against 40.1 ms per sub-integration), else CUDA_CORE. */
+ * runs, the faster of the two on GB300 (16 antennas, nchan 4096, 62500 FFTs, FP16: 14.8
+ * against 24 ms per sub-integration), else CUDA_CORE. */
 enum { GXC_FFT_AUTO = 0, GXC_FFT_CUDA_CORE = 1, GXC_FFT_TENSOR = 2 };
 /* FFT-range split of the FP16 / FP8 tensor-core X-stage: each channel group's FFTs of a block go to
  * two CTAs, the second accumulating into a second plane that finalisation adds.  AUTO: split when
