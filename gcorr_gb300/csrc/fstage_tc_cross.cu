@@ -1,5 +1,5 @@
-// Tensor-core F-stage of handles without autocorrelations: 8192-point windows of 2-bit
-// real data with FP16 or FP8 channelised output, the FFT as two dense DFT products on
+// Tensor-core F-stage of handles without autocorrelations, and of FP8 ones of more than 16
+// antennas: 8192-point windows of 2-bit real data with FP16 or FP8 channelised output, the FFT as two dense DFT products on
 // tcgen05.
 //
 // fstage_tc.cu transforms the same windows in half the time (7.4 against 15.5 ms for 31250

@@ -393,7 +393,9 @@ gxc_status gxc_create(const gxc_config *cfg, gxc_handle **out) {
   // they keep the kernels whose FP32 roundings they have (2-norm of the change otherwise: FP16 at 8192 points 8.5e-5 after
   // 2500 FFTs, at 2048 and 4096 points 1.6e-5; FP8 1e-4 to 1e-3 after 50000)
   const bool cross_only = !cfg->autos && h->chan_type != CHAN_F32;
-  h->tc_cross = h->tc_fstage && cross_only;
+  // Beside autocorrelations the change is about 1e-3 (FP8, 8192 points) or 9e-5 (FP16) times sqrt((nant + 1) / nfft): FP8 over
+  // 50000 FFTs 1.8e-5 with 16 antennas, but 2.0e-5 with 20, which therefore keep the earlier kernel too.
+  h->tc_cross = h->tc_fstage && (cross_only || (h->chan_type == CHAN_F8 && nant > 16));
   if (e == cudaSuccess && h->tc_fstage)
     e = h->tc_cross ? make_fstage_tc_cross_tables(&h->d_tc_tables) : make_fstage_tc_tables(&h->d_tc_tables);
   // otherwise the FP32-accurate F-stage: its first step on tensor cores where that is faster, else the register FFT
