@@ -75,6 +75,7 @@ __device__ __forceinline__ void tc_fence_after() {
 }
 
 __device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t ncols) {
+  __syncwarp();  // by all lanes together; the caller's code before it may branch by lane
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(ncols)
                : "memory");
 }
@@ -211,12 +212,16 @@ __device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uin
 template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 
-// Barrier over the nthreads threads of a warp group of the CTA (id 1..15), and the same with an AND over `ok`.
+// Barrier over the nthreads threads of a warp group of the CTA (id 1..15), and the same with an AND over `ok`.  bar.sync
+// and bar.red are the aligned forms, which all lanes of a warp execute together, and callers arrive from code that branches
+// by lane (waits, ragged loops): the warp converges first.
 __device__ __forceinline__ void group_sync(int id, int nthreads) {
+  __syncwarp();
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 __device__ __forceinline__ bool group_sync_and(int id, int nthreads, bool ok) {
   uint32_t r;
+  __syncwarp();
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.u32 p, %1, 0;\n\t"

@@ -945,6 +945,7 @@ __global__ void __launch_bounds__(NTHREADS_SPLIT, 1) xstage_tc_split_kernel(Para
             make_float2((sm.x + cm.x) / nf, (sm.y + cm.y) / nf);
       }
     }
+    __syncwarp();  // (the loop above ends at different entries within a warp)
     if (p.kparts > 1) cluster.sync();  // no CTA leaves while another reads its shared memory
   } else if (!*(volatile int *)p.err) {  // a timed-out role may have left the staging incomplete
     const float2 *stg = reinterpret_cast<const float2 *>(smem);
