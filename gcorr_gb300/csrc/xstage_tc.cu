@@ -883,8 +883,8 @@ __global__ void __launch_bounds__(NTHREADS_SPLIT, 1) xstage_tc_split_kernel(Para
     // once the last drain is done: every MMA has finished); all threads then add them into the
     // accumulators below, CS consecutive channels of a (baseline, product) contiguous in memory.
     // The register sums W come from D (see above), so V[s1][s2] = (W[s1][s2] + conj(W[s2][s1])) / 2:
-    // one pass stores W[s1][s2] of each output pair, a second adds the other half and scales
-    // (exactly, by a power of two).
+    // one pass stores W[s1][s2] of each output pair, scaled (exactly, by a power of two), a second adds the other half.
+    // Scaled first, the two do not overflow where their mean is finite.
     const float unsc = 0.5f * p.split_unsc;
 #pragma unroll
     for (int pass = 0; pass < 2; pass++) {
@@ -905,8 +905,8 @@ __global__ void __launch_bounds__(NTHREADS_SPLIT, 1) xstage_tc_split_kernel(Para
               float2 *o = reinterpret_cast<float2 *>(smem) +
                           (baseline_index(j, k, p.nant) * 4 + 2 * (u & 1) + (w & 1)) * p.CS + cl;
               const float2 x = acc[G][a][qq];
-              if (pass) *o = make_float2((o->x + x.x) * unsc, (o->y - x.y) * unsc);
-              else *o = x;
+              if (pass) *o = make_float2(fmaf(x.x, unsc, o->x), fmaf(-x.y, unsc, o->y));
+              else *o = make_float2(x.x * unsc, x.y * unsc);
             }
           }
         }
