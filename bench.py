@@ -773,23 +773,8 @@ def main():
         t = tdata.get(key)
         return None if not t else t["per_fft"] * ffts_per_launch + t.get("per_launch_const", 0)
 
-    # the F-stage kernel this FFT length and precision runs
+    fkern = fx.fstage_kernel
     tc_f = f_engine == "tensor"  # the F-stage kernel the handle ran
-    # groups of 16384 samples (from 16384 points on: windows) per SM, the rule of fstage_tc32_worth (csrc/fstage_tc32.cu)
-    groups = -(-fx.fft_block // max(1, 8192 // w.fft_len)) * w.nant / torch.cuda.get_device_properties(0).multi_processor_count
-    if tc_f:
-        fkern = "fstage_tc_kernel"
-    elif not w.is_complex and (2048 <= w.fft_len <= 8192 and groups >= 3 or
-                               w.fft_len >= 16384 and args.precision == "fp32" and groups >= 1):
-        fkern = "fstage_tc32_kernel"
-    elif w.fft_len == 8192:
-        fkern = "fstage_pair_kernel"
-    elif w.fft_len >= 16384 and args.precision != "fp32":
-        fkern = "fstage_h_kernel"
-    elif w.fft_len == 32768:
-        fkern = "fstage_cluster_kernel"
-    else:
-        fkern = "fstage_kernel"
     if f_ms >= x_ms:
         roof = {"kernel": fkern + " (unpack+rotate+FFT+frac-delay)", "bound": "hbm",
                 "achieved": f_bytes / (f_launch_ms / 1e3) / 1e9, "peak": pk["hbm_gbs"], "unit": "GB/s",

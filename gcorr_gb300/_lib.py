@@ -20,7 +20,7 @@ GXC_PRECISION_FP32, GXC_PRECISION_FP16, GXC_PRECISION_FP8 = 0, 1, 2
 GXC_XCORR_NOALLOC_SCRATCH_BYTES = 16 << 20
 GXC_ROTATOR_EXACT, GXC_ROTATOR_FXKERNEL = 0, 1
 GXC_XENGINE_AUTO, GXC_XENGINE_CUDA_CORE, GXC_XENGINE_TENSOR = 0, 1, 2
-GXC_FFT_AUTO, GXC_FFT_CUDA_CORE, GXC_FFT_TENSOR = 0, 1, 2
+GXC_FFT_AUTO, GXC_FFT_CUDA_CORE, GXC_FFT_TENSOR, GXC_FFT_MIXED = 0, 1, 2, 3
 GXC_XSPLIT_AUTO, GXC_XSPLIT_OFF, GXC_XSPLIT_ON = 0, 1, 2
 GXC_FP8_SCALE_CHANNEL, GXC_FP8_SCALE_HANDLE = 0, 1
 _STATUS = {0: "ok", 1: "invalid argument", 2: "unsupported", 3: "CUDA error", 4: "out of memory",
@@ -32,7 +32,7 @@ EXPORTS = [
     "gxc_num_baselines",
     "gxc_status_string", "gxc_create", "gxc_destroy", "gxc_set_input", "gxc_set_delays", "gxc_process",
     "gxc_sync", "gxc_accumulate", "gxc_get_visibilities", "gxc_device_visibilities", "gxc_get_baseline_counts",
-    "gxc_get_valid_flags", "gxc_last_error", "gxc_last_launch_count", "gxc_fft_block", "gxc_num_blocks", "gxc_fft_engine", "gxc_enable_stage_timing",
+    "gxc_get_valid_flags", "gxc_last_error", "gxc_last_launch_count", "gxc_fft_block", "gxc_num_blocks", "gxc_fft_engine", "gxc_fstage_kernel", "gxc_enable_stage_timing",
     "gxc_stage_times", "gxc_xcorr", "gxc_xcorr_noalloc", "gxc_batch_create", "gxc_batch_launch", "gxc_batch_size",
     "gxc_batch_job", "gxc_batch_launch_count", "gxc_batch_destroy", "gxc_pipeline_create", "gxc_pipeline_submit",
     "gxc_pipeline_wait", "gxc_pipeline_sync", "gxc_pipeline_integration", "gxc_pipeline_set_lin2circ",
@@ -152,6 +152,8 @@ def lib():
         l.gxc_num_blocks.restype = C.c_int
         l.gxc_fft_engine.argtypes = [V]
         l.gxc_fft_engine.restype = C.c_int
+        l.gxc_fstage_kernel.argtypes = [V]
+        l.gxc_fstage_kernel.restype = C.c_char_p
         l.gxc_enable_stage_timing.argtypes = [V, C.c_int]
         l.gxc_enable_stage_timing.restype = C.c_int
         l.gxc_stage_times.argtypes = [V, V, V, V]

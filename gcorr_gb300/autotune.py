@@ -1,8 +1,8 @@
 """Autotuner for per-shape launch choices of the correlator.
 
 For one job shape it times process() over the launch plans the shape supports:
-FFT block (FFTs per F/X pass), X-stage engine, F-stage plan (CUDA-core radix FFT
-or tensor-core four-step DFT products) and the X tile's FFT-range split, and
+FFT block (FFTs per F/X pass), X-stage engine, F-stage plan (CUDA-core radix FFT,
+tensor-core four-step DFT products or the FFT with its first step on tensor cores) and the X tile's FFT-range split, and
 keeps the fastest.
 Results are cached on disk (JSON) by shape, so a shape is measured once per
 machine.  Cache file: $GXC_TUNE_CACHE or ~/.cache/gxcorr/tune.json.
@@ -80,7 +80,8 @@ def tune(job: dict, blocks: Iterable[int] = DEFAULT_BLOCKS, engines: Iterable[st
     Coordinate search over the launch plan of one shape:
       1. FFT block T (FFTs per F/X pass) x X engine (tensor cores / CUDA cores);
       2. for the best pair, the F-stage plan (``fft_engine``: CUDA-core radix FFT or tensor-core
-         four-step DFT products, where the shape allows both);
+         four-step DFT products, where the shape allows both; "auto" where it stands for the FFT with
+         its first step on tensor cores);
       3. for a tensor X-stage on FP16 / FP8 data, the X tile's FFT-range split (``x_split`` off / on:
          one or two CTAs per channel group and block).
     Each candidate is the median of `reps` timed process() calls.  Returns {"fft_block",
@@ -96,12 +97,15 @@ def tune(job: dict, blocks: Iterable[int] = DEFAULT_BLOCKS, engines: Iterable[st
     tried = []
     kw = {k: job[k] for k in ("nant", "nchan", "nfft", "nbit", "lo", "bw", "is_complex") if k in job}
 
-    def run(plan):
+    def run(plan, used=None):
         try:
             fx = FxKernel(precision=prec, rotator=job.get("rotator", "exact"), autos=job.get("autos", True), **plan,
                           **kw)
         except Exception:
             return None  # not available for this shape
+        if used and fx.fft_engine_used != used:
+            fx.close()
+            return None
         try:
             fx.setInputData(job["inputs"])
             fx.setDelays(job["poly"], job["fso"])
@@ -113,9 +117,9 @@ def tune(job: dict, blocks: Iterable[int] = DEFAULT_BLOCKS, engines: Iterable[st
 
     best, best_ms = None, None
 
-    def consider(plan):
+    def consider(plan, used=None):
         nonlocal best, best_ms
-        ms = run(plan)
+        ms = run(plan, used)
         if ms is not None and (best_ms is None or ms < best_ms):
             best, best_ms = dict(plan), ms
 
@@ -128,6 +132,7 @@ def tune(job: dict, blocks: Iterable[int] = DEFAULT_BLOCKS, engines: Iterable[st
     for fe in _candidates_f(job, prec):
         if fe != best["fft_engine"]:
             consider(dict(best, fft_engine=fe))
+    consider(dict(best, fft_engine="auto"), used="mixed")
     if best["x_engine"] == "tensor" and prec != "fp32":
         for xs in ("off", "on"):
             consider(dict(best, x_split=xs))

@@ -140,6 +140,12 @@ cudaError_t make_twiddles(int F, float2 **out) {
 
 int fstage_supported(int F) { return F >= 256 && F <= 32768 && (F & (F - 1)) == 0; }
 
+const char *fstage_kernel_name(int log2F, int chan_type) {  // as launch_fstage_l dispatches
+  if (log2F == 13) return "fstage_pair_kernel";
+  if (log2F >= 14 && chan_type != CHAN_F32) return "fstage_h_kernel";
+  return log2F == 15 ? "fstage_cluster_kernel" : "fstage_kernel";
+}
+
 cudaError_t launch_fstage(const Job &job, const float2 *twiddles, int t0, int nt, int T, void *chan, int chan_type,
                           float out_scale, cudaStream_t s, const float *cscale) {
   if (nt <= 0) return cudaSuccess;

@@ -1,5 +1,5 @@
-// Tensor-core assisted F-stage in FP32 accuracy for windows of 2-bit real data: 2048 to 8192 points with every channelised
-// output type, 16384 and 32768 points with FP32 output.
+// Tensor-core assisted F-stage in FP32 accuracy for windows of 2-bit real data: 2048 and 4096 points with every channelised
+// output type, 8192 to 32768 points with FP32 output.
 //
 // Four-step factorisation N = N1 x N2, n = n2 + N2 n1, k = k1 + N1 k2 (fxkernel's dofft,
 // fxkernel/src/fxkernel.cpp:569-580, is the plain unnormalised forward DFT this restates); N2 = 128, at 32768 points 256:
@@ -713,10 +713,10 @@ static cudaError_t launch_t(const Params &p, cudaStream_t s) {
   switch (p.job.log2F) {
     case 11: return launch_l<11, OutT, DBG>(p, s);
     case 12: return launch_l<12, OutT, DBG>(p, s);
-    case 13: return launch_l<13, OutT, DBG>(p, s);
     default: break;
   }
   if constexpr (sizeof(OutT) == 8) {
+    if (p.job.log2F == 13) return launch_l<13, OutT, DBG>(p, s);
     if (p.job.log2F == 14) return launch_l<14, OutT, DBG>(p, s);
     if (p.job.log2F == 15) return launch_l<15, OutT, DBG>(p, s);
   }
@@ -725,14 +725,15 @@ static cudaError_t launch_t(const Params &p, cudaStream_t s) {
 
 }  // namespace f32tc
 
-// 2048 to 8192 points of 2-bit real data, and 16384 and 32768 points with FP32 output (the FP16 and FP8 spectra of
-// those keep fstage_h_kernel, whose FP16 roundings between passes are part of what they are).  At 1024 points, whose rows
+// 2048 and 4096 points of 2-bit real data, and 8192 to 32768 points with FP32 output (FP16 and FP8 spectra of 8192
+// points have fstage_tc_kernel; those of 16384 and 32768 points keep fstage_h_kernel, whose FP16 roundings between passes
+// are part of what they are).  At 1024 points, whose rows
 // hold 8 channels, it measured no faster than the register FFT: 61.4 against 63.5 us for 12 groups per SM.  The
 // rotator's phase must be linear over the samples n2 of a row and over the rows: always so in exact mode, in fxkernel
 // mode when the table split is at N2 samples (8192 and 32768 points).  The output addresses use a 32-bit channel step.
 int fstage_tc32_supported(const Job &job, int T, int chan_type) {
   const int n2 = job.log2F == 15 ? 256 : 128;
-  return !job.is_complex && job.log2F >= 11 && (job.log2F <= 13 || (job.log2F <= 15 && chan_type == CHAN_F32)) &&
+  return !job.is_complex && job.log2F >= 11 && (job.log2F <= 12 || (job.log2F <= 15 && chan_type == CHAN_F32)) &&
          (job.rotator == GXC_ROTATOR_EXACT || job.substride == n2) &&
          (unsigned long long)T * 2 * job.nant * CW * (job.log2F <= 13 ? 4 : 8) * sizeof(float2) <= 0xffffffffull;
 }

@@ -17,6 +17,11 @@
 
 using namespace gxc;
 
+// F-stage kernels of a handle: the register FFT of every shape (fstage.cu), the FP32-accurate one with its first step on
+// tensor cores (fstage_tc32.cu), the tensor-core one of 8192 points (fstage_tc.cu) and its earlier form
+// (fstage_tc_cross.cu).
+enum class FKernel { REGISTER, MIXED, TENSOR, TENSOR_CROSS };
+
 struct gxc_handle {
   gxc_config cfg;
   Job job;
@@ -26,9 +31,7 @@ struct gxc_handle {
   std::vector<std::pair<int, int>> blk;  // blocks of the last process(): (first FFT, FFT count)
   int chan_type = CHAN_F32;
   int xeng = GXC_XENGINE_CUDA_CORE;
-  bool tc_fstage = false;  // tensor-core F-stage (fstage_tc.cu)
-  bool tc_cross = false;   // ... in the form for handles without autocorrelations (fstage_tc_cross.cu)
-  bool tc32_fstage = false;  // FP32-accurate F-stage with its first step on tensor cores (fstage_tc32.cu)
+  FKernel fkern = FKernel::REGISTER;
   void *d_tc_tables = nullptr;
   float out_scale = 1.f;   // applied to channelised values before the cast
   float vis_scale = 1.f;   // 1/out_scale^2, applied at finalisation
@@ -238,7 +241,19 @@ const char *gxc_last_error(const gxc_handle *h) { return h ? h->err.c_str() : "n
 int gxc_last_launch_count(const gxc_handle *h) { return h ? h->launches : 0; }
 int gxc_fft_block(const gxc_handle *h) { return h ? h->T : 0; }
 int gxc_num_blocks(const gxc_handle *h) { return h ? h->nblocks : 0; }
-int gxc_fft_engine(const gxc_handle *h) { return h && h->tc_fstage ? GXC_FFT_TENSOR : GXC_FFT_CUDA_CORE; }
+int gxc_fft_engine(const gxc_handle *h) {
+  if (!h || h->fkern == FKernel::REGISTER) return GXC_FFT_CUDA_CORE;
+  return h->fkern == FKernel::MIXED ? GXC_FFT_MIXED : GXC_FFT_TENSOR;
+}
+const char *gxc_fstage_kernel(const gxc_handle *h) {
+  if (!h) return "";
+  switch (h->fkern) {
+    case FKernel::MIXED: return "fstage_tc32_kernel";
+    case FKernel::TENSOR: return "fstage_tc_kernel";
+    case FKernel::TENSOR_CROSS: return "fstage_tc_cross_kernel";
+    default: return fstage_kernel_name(h->log2F, h->chan_type);
+  }
+}
 const float *gxc_device_visibilities(const gxc_handle *h) { return h ? (const float *)h->d_vis : nullptr; }
 
 static void release(gxc_handle *h) {
@@ -386,20 +401,23 @@ gxc_status gxc_create(const gxc_config *cfg, gxc_handle **out) {
   if (e == cudaSuccess) e = make_twiddles(h->F, &h->d_tw);
   if (e == cudaSuccess) e = make_tile_pairs(nant, &h->d_pairs);
   // AUTO takes the tensor-core F-stage where it runs (8192-point 2-bit real windows, FP16 or
-  // FP8 channelised data): 14.8 ms against 24 ms for the FP32-accurate one per second of the
+  // FP8 channelised data): 14.8 ms against 40 ms for the register FFT per second of the
   // 16-antenna, 512 Ms/s workload at FP16
-  h->tc_fstage = cfg->fft_engine != GXC_FFT_CUDA_CORE && fstage_tc_supported(j, h->chan_type);
+  const bool tensor = cfg->fft_engine != GXC_FFT_CUDA_CORE && fstage_tc_supported(j, h->chan_type);
   // Results without autocorrelations are mostly noise, whose low bits are those of the FP16 or FP8 roundings of the spectra;
   // they keep the kernels whose FP32 roundings they have (2-norm of the change otherwise: FP16 at 8192 points 8.5e-5 after
   // 2500 FFTs, at 2048 and 4096 points 1.6e-5; FP8 1e-4 to 1e-3 after 50000)
   const bool cross_only = !cfg->autos && h->chan_type != CHAN_F32;
   // Beside autocorrelations the change is about 1e-3 (FP8, 8192 points) or 9e-5 (FP16) times sqrt((nant + 1) / nfft): FP8 over
   // 50000 FFTs 1.8e-5 with 16 antennas, but 2.0e-5 with 20, which therefore keep the earlier kernel too.
-  h->tc_cross = h->tc_fstage && (cross_only || (h->chan_type == CHAN_F8 && nant > 16));
-  if (e == cudaSuccess && h->tc_fstage)
-    e = h->tc_cross ? make_fstage_tc_cross_tables(&h->d_tc_tables) : make_fstage_tc_tables(&h->d_tc_tables);
-  // otherwise the FP32-accurate F-stage: its first step on tensor cores where that is faster, else the register FFT
-  h->tc32_fstage = !h->tc_fstage && !cross_only && fstage_tc32_worth(j, h->T, h->chan_type);
+  if (tensor)
+    h->fkern = cross_only || (h->chan_type == CHAN_F8 && nant > 16) ? FKernel::TENSOR_CROSS : FKernel::TENSOR;
+  // otherwise the FP32-accurate F-stage: its first step on tensor cores where that is faster, else the register FFT, which
+  // CUDA_CORE asks for
+  else if (cfg->fft_engine == GXC_FFT_AUTO && !cross_only && fstage_tc32_worth(j, h->T, h->chan_type))
+    h->fkern = FKernel::MIXED;
+  if (e == cudaSuccess && h->fkern == FKernel::TENSOR) e = make_fstage_tc_tables(&h->d_tc_tables);
+  if (e == cudaSuccess && h->fkern == FKernel::TENSOR_CROSS) e = make_fstage_tc_cross_tables(&h->d_tc_tables);
   if (h->chan_type == CHAN_F8 && cfg->fp8_scaling == GXC_FP8_SCALE_CHANNEL) {
     // calibration block: up to 64 FFTs, at most 256 MB of FP32 channelised data (at least 4 FFTs)
     const size_t per_fft32 = (size_t)cfg->nchan * 2 * nant * sizeof(float2);
@@ -642,6 +660,22 @@ gxc_status gxc_process(gxc_handle *h, void *stream) { return gxc::process_chaine
 
 // process() with its host->device input copies ordered behind copy_wait (when given) and
 // followed by a record of copy_done (when given); batches use it to chain the jobs' copies.
+// FFTs [t0, t0 + nt) through the handle's F-stage kernel into chan; probe as for launch_fstage_tc
+static cudaError_t run_fstage(const gxc_handle *h, int t0, int nt, void *chan, float out_scale, cudaStream_t s,
+                              const float *cscale, float2 *probe) {
+  switch (h->fkern) {
+    case FKernel::MIXED:
+      return launch_fstage_tc32(h->job, t0, nt, h->T, chan, h->chan_type, out_scale, s, cscale, probe);
+    case FKernel::TENSOR:
+      return launch_fstage_tc(h->job, h->d_tc_tables, t0, nt, h->T, chan, h->chan_type, out_scale, s, cscale, probe);
+    case FKernel::TENSOR_CROSS:
+      return launch_fstage_tc_cross(h->job, h->d_tc_tables, t0, nt, h->T, chan, h->chan_type, out_scale, s, cscale, probe);
+    default:
+      return probe ? launch_fstage_probe(h->job, h->d_tw, t0, nt, h->T, chan, h->chan_type, out_scale, probe, s)
+                   : launch_fstage(h->job, h->d_tw, t0, nt, h->T, chan, h->chan_type, out_scale, s, cscale);
+  }
+}
+
 extern "C++" gxc_status gxc::process_chained(gxc_handle *h, void *stream, cudaEvent_t copy_wait,
                                              cudaEvent_t copy_done, int nchunk, const cudaEvent_t *chunk_ev,
                                              const long long *chunk_end) {
@@ -774,17 +808,7 @@ extern "C++" gxc_status gxc::process_chained(gxc_handle *h, void *stream, cudaEv
     // with per-channel FP8 scales the channel's scale replaces the handle's
     const float osc = h->d_cscale ? 1.0f : h->out_scale;
     if (timing) GXC_CUDA(h, cudaEventRecord(h->ev_stage[3 * b], s), "timing event");
-    if (h->tc_fstage)
-      GXC_CUDA(h,
-               (h->tc_cross ? launch_fstage_tc_cross : launch_fstage_tc)(h->job, h->d_tc_tables, t0, nt, h->T, h->d_chan,
-                                                                         h->chan_type, osc, s, h->d_cscale, nullptr),
-               "tensor-core F-stage kernel");
-    else if (h->tc32_fstage)
-      GXC_CUDA(h, launch_fstage_tc32(h->job, t0, nt, h->T, h->d_chan, h->chan_type, osc, s, h->d_cscale),
-               "tensor-core assisted F-stage kernel");
-    else
-      GXC_CUDA(h, launch_fstage(h->job, h->d_tw, t0, nt, h->T, h->d_chan, h->chan_type, osc, s, h->d_cscale),
-               "F-stage kernel");
+    GXC_CUDA(h, run_fstage(h, t0, nt, h->d_chan, osc, s, h->d_cscale, nullptr), "F-stage kernel");
     launches++;
     if (timing) GXC_CUDA(h, cudaEventRecord(h->ev_stage[3 * b + 1], s), "timing event");
     if (h->nbl > 0) {
@@ -842,12 +866,7 @@ gxc_status gxc_probe_unpack(gxc_handle *h, float *decoded) {
     const int t0 = b * h->T;
     const int nt = (c.nfft - t0) < h->T ? (c.nfft - t0) : h->T;
     // the probe runs the handle's own F-stage kernel family
-    e = h->tc_fstage ? (h->tc_cross ? launch_fstage_tc_cross : launch_fstage_tc)(
-                           h->job, h->d_tc_tables, t0, nt, h->T, chan, h->chan_type, h->out_scale, nullptr, nullptr, probe)
-        : h->tc32_fstage ? launch_fstage_tc32(h->job, t0, nt, h->T, chan, h->chan_type, h->out_scale, nullptr, nullptr,
-                                              probe)
-                     : launch_fstage_probe(h->job, h->d_tw, t0, nt, h->T, chan, h->chan_type, h->out_scale, probe,
-                                           nullptr);
+    e = run_fstage(h, t0, nt, chan, h->out_scale, nullptr, nullptr, probe);
   }
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e == cudaSuccess) e = cudaMemcpy(decoded, probe, n * sizeof(float2), cudaMemcpyDefault);
@@ -868,16 +887,14 @@ gxc_status gxc_sync(gxc_handle *h) {
     GXC_CUDA(h, xstage_tensor_take_error(&flag), "reading the X-stage status");
     if (flag) return fail(h, GXC_ERR_TIMEOUT, "tensor-core X-stage: a bounded device wait expired");
   }
-  if (h->tc_fstage) {
+  if (h->fkern != FKernel::REGISTER) {
     int flag = 0;
-    GXC_CUDA(h, h->tc_cross ? fstage_tc_cross_take_error(&flag) : fstage_tc_take_error(&flag),
+    GXC_CUDA(h,
+             h->fkern == FKernel::MIXED    ? fstage_tc32_take_error(&flag)
+             : h->fkern == FKernel::TENSOR ? fstage_tc_take_error(&flag)
+                                           : fstage_tc_cross_take_error(&flag),
              "reading the F-stage status");
-    if (flag) return fail(h, GXC_ERR_TIMEOUT, "tensor-core F-stage: a bounded device wait expired");
-  }
-  if (h->tc32_fstage) {
-    int flag = 0;
-    GXC_CUDA(h, fstage_tc32_take_error(&flag), "reading the F-stage status");
-    if (flag) return fail(h, GXC_ERR_TIMEOUT, "tensor-core assisted F-stage: a bounded device wait expired");
+    if (flag) return fail(h, GXC_ERR_TIMEOUT, std::string(gxc_fstage_kernel(h)) + ": a bounded device wait expired");
   }
   return GXC_OK;
 }

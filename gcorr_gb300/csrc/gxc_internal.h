@@ -91,6 +91,9 @@ cudaError_t launch_fstage_tc(const Job &job, const void *tables, int t0, int nt,
                              float2 *probe = nullptr);
 cudaError_t fstage_tc_take_error(int *flag);
 
+// Name of the kernel that launch_fstage runs at 2^log2F points.
+const char *fstage_kernel_name(int log2F, int chan_type);
+
 // fstage_tc_cross.cu: the same for handles without autocorrelations, and FP8 ones of more than 16 antennas (its own
 // constant operands).
 cudaError_t make_fstage_tc_cross_tables(void **out);
@@ -99,8 +102,8 @@ cudaError_t launch_fstage_tc_cross(const Job &job, const void *tables, int t0, i
                                    float2 *probe = nullptr);
 cudaError_t fstage_tc_cross_take_error(int *flag);
 
-// fstage_tc32.cu: the F-stage in FP32 accuracy with its first step on tensor cores (2-bit real windows; 2048 to 8192 points
-// with every channelised type, 16384 and 32768 points with FP32).  T: the handle's FFT block.  probe as for launch_fstage_tc.
+// fstage_tc32.cu: the F-stage in FP32 accuracy with its first step on tensor cores (2-bit real windows; 2048 and 4096
+// points with every channelised type, 8192 to 32768 points with FP32).  T: the handle's FFT block.  probe as for launch_fstage_tc.
 int fstage_tc32_supported(const Job &job, int T, int chan_type);
 int fstage_tc32_worth(const Job &job, int T, int chan_type);  // supported, and faster than the register FFT at this size
 cudaError_t launch_fstage_tc32(const Job &job, int t0, int nt, int T, void *chan, int chan_type, float out_scale,

@@ -194,8 +194,13 @@ class FxKernel:
 
     @property
     def fft_engine_used(self) -> str:
-        """The F-stage engine this handle runs ("tensor" or "cuda_core"; "auto" resolved)."""
-        return "tensor" if L.lib().gxc_fft_engine(self._h) == L.GXC_FFT_TENSOR else "cuda_core"
+        """The F-stage engine this handle runs ("tensor", "mixed" or "cuda_core"; "auto" resolved)."""
+        return {L.GXC_FFT_TENSOR: "tensor", L.GXC_FFT_MIXED: "mixed"}.get(L.lib().gxc_fft_engine(self._h), "cuda_core")
+
+    @property
+    def fstage_kernel(self) -> str:
+        """Name of the F-stage kernel this handle runs."""
+        return L.lib().gxc_fstage_kernel(self._h).decode()
 
     @property
     def num_blocks(self) -> int:

@@ -59,12 +59,13 @@ enum { GXC_XENGINE_AUTO = 0, GXC_XENGINE_CUDA_CORE = 1, GXC_XENGINE_TENSOR = 2 }
 /* F-stage FFT engine.  TENSOR: the FFT as two dense DFT products on tcgen05 (FP16
  * operands, FP32 accumulation), for FP16 / FP8 channelised output of 8192-point
  * windows of 2-bit real data (nchan 4096); it adds four FP16 roundings inside the
- * FFT.  CUDA_CORE: the FP32-accurate FFT of every shape (FP32
- * arithmetic; for larger blocks of 2-bit real windows of 2048 points and more the
- * first step, whose inputs are exact, runs on tensor cores).  AUTO: TENSOR where it
- * runs, the faster of the two on GB300 (16 antennas, nchan 4096, 62500 FFTs, FP16: 14.8
- * against 24 ms per sub-integration), else CUDA_CORE. */
-enum { GXC_FFT_AUTO = 0, GXC_FFT_CUDA_CORE = 1, GXC_FFT_TENSOR = 2 };
+ * FFT.  CUDA_CORE: the FP32 register FFT of every shape.  AUTO: TENSOR where it
+ * runs (16 antennas, nchan 4096, 62500 FFTs, FP16: 14.8 ms per sub-integration, 40 for
+ * CUDA_CORE), else MIXED where it is faster, else CUDA_CORE.  MIXED, an answer of
+ * gxc_fft_engine and not a choice: the FFT in FP32 accuracy with its first step on
+ * tensor cores, for blocks of 2-bit real windows of 2048 points and more that fill the
+ * GPU (the same workload in FP32: 24.3 against 40.8 ms). */
+enum { GXC_FFT_AUTO = 0, GXC_FFT_CUDA_CORE = 1, GXC_FFT_TENSOR = 2, GXC_FFT_MIXED = 3 };
 /* FFT-range split of the FP16 / FP8 tensor-core X-stage: each channel group's FFTs of a block go to
  * two CTAs, the second accumulating into a second plane that finalisation adds.  AUTO: split when
  * the channel groups are fewer than the SMs.  OFF: never.  ON: whenever the block holds at least
@@ -181,8 +182,10 @@ int gxc_fft_block(const gxc_handle *h);
    host and the block was chosen, the passes cover 4096, 8192, ... FFTs up to the block (the
    compute starts after a shorter copy), which can add passes. */
 int gxc_num_blocks(const gxc_handle *h);
-/* F-stage engine this handle runs: GXC_FFT_TENSOR or GXC_FFT_CUDA_CORE (AUTO resolved). */
+/* F-stage engine this handle runs: GXC_FFT_TENSOR, GXC_FFT_MIXED or GXC_FFT_CUDA_CORE (AUTO resolved). */
 int gxc_fft_engine(const gxc_handle *h);
+/* Name of the F-stage kernel this handle runs (a static string). */
+const char *gxc_fstage_kernel(const gxc_handle *h);
 
 /* Stage timing: when enabled, process() records CUDA events around the F-stage
  * and X-stage launches; gxc_stage_times returns the summed milliseconds of the
