@@ -153,7 +153,7 @@ struct FParams {
 
 // Fringe rotator exp(-2 pi i (m c + b)) for a whole number m.  EXACT (FP32 spectra from 8192 points on): the rounding of
 // m c, which is large in turns at steep delay rates, and the low parts of c and b enter as a small rotation.  Without
-// them a delay rate of 5e-4 (256 Ms/s, 8192 points) cost 1.2e-5 of a product, now 3e-7; the spectra in FP16 and FP8 round
+// them a delay rate of 5e-4 (256 Ms/s) cost 2.2e-5 of a product at 8192 points, 1.0e-4 at 32768, now 3e-7; the spectra in FP16 and FP8 round
 // more coarsely and keep the plain argument.
 template <bool EXACT>
 __device__ __forceinline__ float2 rotator(float m, float c, float c_lo, float b, float b_lo) {

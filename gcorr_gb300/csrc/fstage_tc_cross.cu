@@ -1,9 +1,8 @@
-// Tensor-core F-stage of handles without autocorrelations, and of FP8 ones of more than 16
-// antennas: 8192-point windows of 2-bit real data with FP16 or FP8 channelised output, the FFT as two dense DFT products on
-// tcgen05.
+// Tensor-core F-stage of handles without autocorrelations: 8192-point windows of 2-bit real data with FP16 or FP8
+// channelised output, the FFT as two dense DFT products on tcgen05.
 //
 // fstage_tc.cu transforms the same windows in half the time (7.4 against 15.5 ms for 31250
-// FFTs of 16 antennas), with other FP32 roundings before the FP16 ones.  Beside
+// FFTs of 16 antennas) and with the same error, but with other FP32 roundings before the FP16 ones.  Beside
 // autocorrelations the difference is 6e-6 of a result's 2-norm after 2500 FFTs; in a result
 // of cross products alone, which is mostly noise, it is 8.5e-5 (FP8, 50000 FFTs: 9.6e-4).
 // Such results are kept as they are by keeping this kernel for them.

@@ -404,17 +404,17 @@ gxc_status gxc_create(const gxc_config *cfg, gxc_handle **out) {
   // FP8 channelised data): 14.8 ms against 40 ms for the register FFT per second of the
   // 16-antenna, 512 Ms/s workload at FP16
   const bool tensor = cfg->fft_engine != GXC_FFT_CUDA_CORE && fstage_tc_supported(j, h->chan_type);
-  // Results without autocorrelations are mostly noise, whose low bits are those of the FP16 or FP8 roundings of the spectra;
-  // they keep the kernels whose FP32 roundings they have (2-norm of the change otherwise: FP16 at 8192 points 8.5e-5 after
-  // 2500 FFTs, at 2048 and 4096 points 1.6e-5; FP8 1e-4 to 1e-3 after 50000)
-  const bool cross_only = !cfg->autos && h->chan_type != CHAN_F32;
-  // Beside autocorrelations the change is about 1e-3 (FP8, 8192 points) or 9e-5 (FP16) times sqrt((nant + 1) / nfft): FP8 over
-  // 50000 FFTs 1.8e-5 with 16 antennas, but 2.0e-5 with 20, which therefore keep the earlier kernel too.
+  // fstage_tc.cu and fstage_tc_cross.cu, and the mixed kernel and the register FFT, differ in FP32 roundings that flip some of
+  // the FP16 or FP8 roundings after them.  The errors against 64 bits are the same; products of noise move by 8.5e-5 (FP16)
+  // and 9.6e-4 (FP8) of their 2-norm between the first two, by 1.5e-5 and 1.9e-4 between the others, and a whole result with
+  // autocorrelations by sqrt((nant + 1) / nfft) of that.  A result of cross products alone has nothing beside that noise:
+  // there the kernels that would move it by more than 2e-5 give way to those whose roundings such results have always had.
   if (tensor)
-    h->fkern = cross_only || (h->chan_type == CHAN_F8 && nant > 16) ? FKernel::TENSOR_CROSS : FKernel::TENSOR;
+    h->fkern = cfg->autos ? FKernel::TENSOR : FKernel::TENSOR_CROSS;
   // otherwise the FP32-accurate F-stage: its first step on tensor cores where that is faster, else the register FFT, which
   // CUDA_CORE asks for
-  else if (cfg->fft_engine == GXC_FFT_AUTO && !cross_only && fstage_tc32_worth(j, h->T, h->chan_type))
+  else if (cfg->fft_engine == GXC_FFT_AUTO && (cfg->autos || h->chan_type != CHAN_F8) &&
+           fstage_tc32_worth(j, h->T, h->chan_type))
     h->fkern = FKernel::MIXED;
   if (e == cudaSuccess && h->fkern == FKernel::TENSOR) e = make_fstage_tc_tables(&h->d_tc_tables);
   if (e == cudaSuccess && h->fkern == FKernel::TENSOR_CROSS) e = make_fstage_tc_cross_tables(&h->d_tc_tables);

@@ -94,8 +94,7 @@ cudaError_t fstage_tc_take_error(int *flag);
 // Name of the kernel that launch_fstage runs at 2^log2F points.
 const char *fstage_kernel_name(int log2F, int chan_type);
 
-// fstage_tc_cross.cu: the same for handles without autocorrelations, and FP8 ones of more than 16 antennas (its own
-// constant operands).
+// fstage_tc_cross.cu: the same for handles without autocorrelations (its own constant operands).
 cudaError_t make_fstage_tc_cross_tables(void **out);
 cudaError_t launch_fstage_tc_cross(const Job &job, const void *tables, int t0, int nt, int T, void *chan, int chan_type,
                                    float out_scale, cudaStream_t s, const float *cscale = nullptr,

@@ -44,9 +44,20 @@ def test_fp32_lines(nchan, register):
 def test_fp16_and_fp8_engines(precision):
     assert _kernel(4, 4096, 3000, precision) == ("tensor", "fstage_tc_kernel")
     assert _kernel(4, 4096, 3000, precision, fft_engine="cuda_core") == ("cuda_core", "fstage_pair_kernel")
+    assert _kernel(4, 4096, 3000, precision, autos=False) == ("tensor", "fstage_tc_cross_kernel")
     assert _kernel(4, 1024, 10000, precision) == ("mixed", "fstage_tc32_kernel")
     assert _kernel(4, 1024, 10000, precision, fft_engine="cuda_core") == ("cuda_core", "fstage_kernel")
     assert _kernel(4, 8192, 3000, precision) == ("cuda_core", "fstage_h_kernel")
+
+
+@pytest.mark.parametrize("precision", ["fp16", "fp8"])
+@pytest.mark.parametrize("nchan", [1024, 4096])
+def test_choice_does_not_hang_on_the_antenna_count(nchan, precision):
+    """Whatever the number of antennas: the same kernel for handles with autocorrelations, and one without."""
+    for autos, kernels in ((True, {"fstage_tc_kernel" if nchan == 4096 else "fstage_tc32_kernel"}),
+                           (False, {"fstage_tc_cross_kernel" if nchan == 4096 else
+                                    "fstage_tc32_kernel" if precision == "fp16" else "fstage_kernel"})):
+        assert {_kernel(n, nchan, 2000, precision, autos=autos)[1] for n in (2, 16, 17, 20, 64)} == kernels
 
 
 @pytest.mark.parametrize("nchan", [1024, 4096, 16384])
