@@ -8,12 +8,19 @@
 // D1 (rows (window, k1), 64 of them; columns n2) = A1 B1^T per polarisation, real and imaginary part, K = (window,
 // n1).  The fringe rotator of sample n is exp(-2 pi i (c0 + c1 n)): its n1 part is folded into A1 (rows k1 of
 // window w: W_N1^(n1 k1) e^(-2 pi i 128 n1 c1), block-diagonal over the 64 / N1 windows of a group), its n2 part into
-// the twiddles of step 2.  A1 is split into FP16 hi and lo halves (22 significand bits).  B1 holds the levels times
-// 1039: 1039 and 3466 are FP16 values, and 3466 / 1039 is 3.3359 to 2.9e-8 (3.3359f is off by 2.0e-8, half a unit of its
-// last bit being 3.6e-8).  D1 = A_lo B + A_hi B, in this order: the small terms first, so that tensor memory's rounding
-// toward zero acts on the sum only four times.  An exact hi and lo pair of levels (3.3359375 - 628 x 2^-24) took half as
-// many MMAs again and twice the decode's stores, 25.1 against 24.2 ms (16 antennas, 62500 FFTs), for the same error:
-// power spectra 2.3e-7 rms from FP64 at 8192 points, 3.1e-7 at 4096, 4.1e-7 at 2048.
+// the twiddles of step 2.  A1 is split into FP16 hi and lo halves (23 significand bits; the FP32 product that they hold is
+// itself off by about a unit of the 24th).  B1 holds the levels as 1039 and 3466, FP16 values that stand for the FP32 levels
+// to less than half a unit of their last bit (kUnit).  D1 = A_lo B + A_hi B, in this order: the small terms first, so that
+// tensor memory's rounding toward zero acts on the large sum only once per K step of A_hi (one, two and four with terms at
+// 2048, 4096 and 8192 points, eight beyond); what it takes away on average is in A1 (Plan::RZ).  An exact hi and lo pair of
+// levels (3.3359375 - 628 x 2^-24) took half as many MMAs again and twice the decode's stores, 25.1 against 24.2 ms (16
+// antennas, 62500 FFTs), and products of 48 bits in A1 24.5 -> 25.8 ms for 1 % less error.
+//
+// Error against FP64, FP32 sums of 32, 16, 8, 4 and 4 FFTs (2048 to 32768 points; 57 and 38 antennas, 256 MHz), with that of
+// the register FFT as it was when this kernel took its place: power spectra 1.54, 1.39, 1.50, 2.05, 2.12e-7 rms (1.71, 1.65,
+// 1.48, 2.46, 2.27e-7), of which the mean is 0.1e-7 (1.1, 1.1, 0.8, 1.5, 1.0e-7); cross products 2.5, 2.4, 2.4, 2.6, 2.7e-7
+// (3.1, 3.1, 2.9, 3.2, 3.3e-7), and at 32 MHz, where the fringe turns further in a window, 2.6, 2.5, 2.5, 2.7, 2.7e-7 (3.3,
+// 3.5, 4.5, 7.0, 13e-7).
 // Step 2, the N2-point DFTs over n2, runs on the CUDA cores in FP32: a thread owns one row, so the transform needs no
 // exchange between threads.  Radix 8 over j (n2 = i + (N2 / 8) j), back to tensor memory, radix N2 / 8 over i.  With
 // theta = k1 / N + c1 both passes take their twiddles as powers of e^(-2 pi i theta) (the DFT at a shifted
@@ -37,7 +44,7 @@
 // and A1 (128 KB) is single, shared by both polarisations and by all windows of the same slope.  At 16384 points team and
 // slot s belong to polarisation s.  At 32768 points D1 takes all of tensor memory: eight transform warps of 144 registers
 // (radix 32 holds 16 packed pairs) alternate with the MMAs (4,300 clocks of about 22,000 per window and polarisation).
-// F-stage, 10 antennas, 32768 points, 3901 FFTs: 5.80 ms, 15.85 for the cluster kernel; error of the crosses 4.2e-7 (1.0e-6).
+// F-stage, 10 antennas, 32768 points, 3901 FFTs: 5.80 ms, 15.85 for the cluster kernel.
 //
 // Every wait is bounded; on expiry the kernel sets an error flag (read by gxc_sync as GXC_ERR_TIMEOUT), lets issued
 // MMAs drain, frees tensor memory and returns.
@@ -71,6 +78,10 @@ struct Plan {
   static constexpr int NP = N2 == 128 ? 7 : 8, ES = N2 == 128 ? 8 : 16;  // log2 N2; e entries of a window
   static constexpr int NPR = N2 / 16;         // pairs of samples i, i + 1
   static constexpr int NR = L == 15 ? 2 : 4;  // table ring
+  // Tensor memory rounds its FP32 sums toward zero, which leaves D1 low by this much on average (a row has terms in one,
+  // two, four or eight K steps); A1's lo half carries the inverse.  Measured on sampled noise: with it power spectra are
+  // within 2e-8 of FP64 on average, at each length.
+  static constexpr float RZ = L == 11 ? 1.04e-7f : L == 12 ? 1.13e-7f : L == 13 ? 1.39e-7f : L == 14 ? 2.0e-7f : 2.05e-7f;
   // ring entry (float2): fsub[(w, k1)], e[w][ES] (e^(-2 pi i 2^s c1), s < NP; e^(-2 pi i c0), or 0 for a flagged
   // window), fst[w][k2] = e^(2 pi i N1 k2 cf) * scale
   static constexpr int T_FSUB = 0, T_E = ROWS, T_FST = T_E + ES * NW, TAB = T_FST + NK2 * NW;
@@ -103,13 +114,13 @@ struct Params {
 
 __device__ int g_f32tc_err;
 
-// Tensor memory rounds its FP32 sums toward zero, which leaves the spectra low, and 3466 / 1039 is 4.9e-8 below 3.3359f;
-// A1's lo half carries the inverse.  Measured: with 9.5e-8 power spectra come out 1.5e-7 low on average, with this
-// value within 0.2e-7 (2048 to 8192 points).
-constexpr float kRz = 1.7e-7f;
-
-// A1 carries 2^10 / 1039 (FP16 holds it well), the frac-delay table 2^-10.
-constexpr float kScale = 1024.0f / 1039.0f;
+// The operand levels 1039 and 3466 stand for 1039 kUnit and 3466 kUnit, which are 1 + 4.1e-8 and 3.3359f (1 - 0.8e-8): both
+// round to the FP32 level.  (Their ratio is 4.9e-8 short of 3.3359f; the high level, which carries most of the power of
+// sampled noise, is the nearer one.)
+constexpr double kUnit = (1.0 + 4.1e-8) / 1039.0;
+// A1 carries kUnit 2^14, so that its lo half stays in FP16's normal range; the frac-delay table carries 2^-14.  kScale holds
+// it in FP32, kLevel the rest, which goes into the lo half.
+constexpr float kScale = (float)(kUnit * 16384.0), kLevel = (float)(kUnit * 16384.0 / (double)kScale - 1.0);
 
 // Tensor-memory column (= row of B1) of sample n2 = i + (N2 / 8) j (j < 8): 16 pr + 2 (j xor pr / 2) + (i mod 2) with
 // pr = i / 2.  Samples i, i + 1 are adjacent columns, the lanes of packed FP32 pairs, and the eight j of a pair are 16
@@ -510,7 +521,7 @@ __global__ void __launch_bounds__(Plan<L>::NT, 1) fstage_tc32_kernel(Params p) {
         } else {
           const int y = x - P::T_FST;
           arg = 2.0f * ((float)(N1 * (y % P::NK2)) * gg[y / P::NK2].cf);
-          sc = p.out_scale * 0x1p-10f;  // powers of two: exact
+          sc = p.out_scale * 0x1p-14f;  // powers of two: exact
         }
         float sn, cs;
         sincospif(arg, &sn, &cs);
@@ -578,8 +589,7 @@ __global__ void __launch_bounds__(Plan<L>::NT, 1) fstage_tc32_kernel(Params p) {
             for (int j = 0; j < 8; j++) {
               const uint32_t hb = j < 4 ? h0[j >> 1] : h1[(j - 4) >> 1];
               const float2 hf = __half22float2(*reinterpret_cast<const __half2 *>(&hb));
-              const float v = (j & 1) ? hf.y : hf.x;
-              pr[N2 * ((8 * o) % N1 + j)] = make_float2(copysignf(fabsf(v) > 2000.0f ? 3.3359f : 1.0f, v), 0.f);
+              pr[N2 * ((8 * o) % N1 + j)] = make_float2((float)((double)((j & 1) ? hf.y : hf.x) * kUnit), 0.f);
             }
           }
         }
@@ -601,8 +611,9 @@ __global__ void __launch_bounds__(Plan<L>::NT, 1) fstage_tc32_kernel(Params p) {
             const float2 fr = __half22float2(xr), fi = __half22float2(xi);
             hr[e] = *reinterpret_cast<const uint32_t *>(&xr);
             hi[e] = *reinterpret_cast<const uint32_t *>(&xi);
-            lr[e] = pack_h2(fmaf(a.x, kRz, a.x - fr.x), fmaf(b.x, kRz, b.x - fr.y));
-            li[e] = pack_h2(fmaf(a.y, kRz, a.y - fi.x), fmaf(b.y, kRz, b.y - fi.y));
+            constexpr float up = kLevel + P::RZ;
+            lr[e] = pack_h2(fmaf(a.x, up, a.x - fr.x), fmaf(b.x, up, b.x - fr.y));
+            li[e] = pack_h2(fmaf(a.y, up, a.y - fi.x), fmaf(b.y, up, b.y - fi.y));
           }
           const int ch = w * (N1 / 8) + cc;
           unsigned char *dst = a1 + (ch >> 3) * (ROWS * 128) + r * 128 + (((ch & 7) ^ (r & 7)) << 4);
