@@ -52,15 +52,11 @@
 #include "gxc_internal.h"
 #include "tcgen05_util.cuh"
 
-#include <math.h>
-#include <vector>
-
 namespace gxc {
 
 namespace f32tc {
 
 constexpr int DW = 8, GT = DW * 32;          // decode warps and threads
-constexpr int KB = 128 * 128;                // SW128 K-block of 128 rows (64 FP16 K-elements)
 
 template <int L>
 struct Plan {

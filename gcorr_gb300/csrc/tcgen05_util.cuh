@@ -196,17 +196,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// D[tmem] (+)= A[tmem] * B[smem]^T, kind::f16: A's row i is tensor-memory lane i, two FP16 K-elements per column.
-__device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
-                                           uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
 // Register share of this warpgroup (4 warps, all of which execute it); the shares of a block's warpgroups add up to
 // at most what it was launched with.
 template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
@@ -247,7 +236,8 @@ __device__ __forceinline__ uint64_t desc_sw128(uint32_t saddr) {
 
 // The same descriptor as two words: the address word, to which the offset of a K step or block is added (>> 4), and a
 // constant.  An MMA-issuing thread then spends one add per operand instead of building 64-bit descriptors, which held
-// its MMAs apart (about 120 clocks each where the tensor pipe takes 64).
+// its MMAs apart (about 120 clocks each where the tensor pipe takes 64).  mma_f16_ts_lo: A from tensor memory, its row i in
+// lane i, two FP16 K-elements per column.
 constexpr uint32_t DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
 __device__ __forceinline__ uint32_t desc_lo(uint32_t saddr) { return ((saddr & 0x3FFFFu) >> 4) | (1u << 16); }
 template <bool ACC>

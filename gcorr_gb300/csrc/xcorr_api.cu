@@ -45,16 +45,16 @@ __global__ void divide_kernel(const float2 *__restrict__ vsum, const float2 *__r
   out[i] = make_float2((s.x + c.x) / nfft, (s.y + c.y) / nfft);
 }
 
-// local: plain device memory of the current device.
-bool is_device(const void *p, bool *local) {
+// local (where asked for): plain device memory of the current device.
+bool is_device(const void *p, bool *local = nullptr) {
   cudaPointerAttributes a;
-  *local = false;
+  if (local) *local = false;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
   int dev = -1;
-  *local = a.type == cudaMemoryTypeDevice && cudaGetDevice(&dev) == cudaSuccess && a.device == dev;
+  if (local) *local = a.type == cudaMemoryTypeDevice && cudaGetDevice(&dev) == cudaSuccess && a.device == dev;
   return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
@@ -146,8 +146,8 @@ extern "C" gxc_status gxc_xcorr(const float *ants, int nant, int nfft, int nchan
   void *chan = nullptr;
   float2 *vsum = nullptr, *vcomp = nullptr, *dants = nullptr, *dout = nullptr;
   int2 *pairs = nullptr;
-  bool ants_local, out_local;
-  const bool ants_dev = is_device(ants, &ants_local), out_dev = is_device(accum, &out_local);
+  bool ants_local;
+  const bool ants_dev = is_device(ants, &ants_local), out_dev = is_device(accum);
   cudaError_t e = cudaSuccess;
   if (!ants_dev) e = cudaMalloc((void **)&dants, nin * sizeof(float2));
   if (e == cudaSuccess && !out_dev) e = cudaMalloc((void **)&dout, nvis * sizeof(float2) + 16);

@@ -39,3 +39,18 @@ def test_every_aligned_instruction_is_in_a_wrapper():
 @pytest.mark.parametrize("file,name,body", _aligned_wrappers(), ids=lambda v: v if isinstance(v, str) and len(v) < 40 else "")
 def test_warp_converges_before_an_aligned_instruction(file, name, body):
     assert "__syncwarp();" in body[:ALIGNED.search(body).start()], f"{file}: {name}"
+
+
+def test_every_shared_device_helper_has_a_caller():
+    """The helpers and constants of tcgen05_util.cuh, and the constants of the F-stage sources, are used."""
+    text = {}
+    for f in sorted(os.listdir(CSRC)):
+        if f.endswith((".cu", ".cuh")):
+            with open(os.path.join(CSRC, f)) as h:
+                text[f] = re.sub(r"//[^\n]*", "", h.read())
+    names = re.findall(r"__device__ __forceinline__ \w+ (\w+)\(", text["tcgen05_util.cuh"])
+    unused = [n for n in names if len(re.findall(r"\b%s\b" % n, "".join(text.values()))) < 2]
+    for f, t in text.items():
+        unused += [f + ": " + n for n in re.findall(r"\bconstexpr (?:int|float|double|uint32_t) (\w+) =", t)
+                   if len(re.findall(r"\b%s\b" % n, "".join(text.values()) if f.endswith(".cuh") else t)) < 2]
+    assert not unused
