@@ -778,7 +778,7 @@ def main():
     if f_ms >= x_ms:
         roof = {"kernel": fkern + " (unpack+rotate+FFT+frac-delay)", "bound": "hbm",
                 "achieved": f_bytes / (f_launch_ms / 1e3) / 1e9, "peak": pk["hbm_gbs"], "unit": "GB/s",
-                "traffic": traffic("fstage_tc_kernel" if tc_f else "fstage_kernel"),
+                "traffic": traffic(fkern),
                 "algorithmic_bytes_per_launch": f_bytes,
                 "launch_ms": f_launch_ms, "launches_per_step": nlaunch, "ffts_per_launch": ffts_per_launch,
                 "fft_tflops": fftflops / (f_ms / 1e3) / 1e12, "fp32_peak_tflops_nominal": fp32_peak}
