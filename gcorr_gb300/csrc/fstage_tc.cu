@@ -620,9 +620,7 @@ cudaError_t launch_fstage_tc(const Job &job, const void *tables, int t0, int nt,
   if (e != cudaSuccess) return e;
   const long long nwin = (long long)nt * job.nant;
   const unsigned grid = (unsigned)(nwin < nsm ? nwin : nsm);
-  // the output role forms k2 * step (step = the bytes of four channel tiles) with a 32-bit step
-  if ((unsigned long long)T * 2 * job.nant * CW * 4 * chan_elem_bytes(chan_type) > 0xffffffffull)
-    return cudaErrorInvalidValue;
+  if (!fstage_tc_addresses(job.nant, T, chan_type)) return cudaErrorInvalidValue;
   auto launch = [&](auto kern) -> cudaError_t {
     cudaError_t e2 = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     if (e2 != cudaSuccess) return e2;

@@ -410,7 +410,7 @@ gxc_status gxc_create(const gxc_config *cfg, gxc_handle **out) {
   // autocorrelations by sqrt((nant + 1) / nfft) of that.  A result of cross products alone has nothing beside that noise:
   // there the kernels that would move it by more than 2e-5 give way to those whose roundings such results have always had.
   if (tensor)
-    h->fkern = cfg->autos ? FKernel::TENSOR : FKernel::TENSOR_CROSS;
+    h->fkern = cfg->autos && fstage_tc_addresses(nant, h->T, h->chan_type) ? FKernel::TENSOR : FKernel::TENSOR_CROSS;
   // otherwise the FP32-accurate F-stage: its first step on tensor cores where that is faster, else the register FFT, which
   // CUDA_CORE asks for
   else if (cfg->fft_engine == GXC_FFT_AUTO && (cfg->autos || h->chan_type != CHAN_F8) &&

@@ -84,6 +84,11 @@ cudaError_t launch_fstage_probe(const Job &job, const float2 *twiddles, int t0, 
 
 // fstage_tc.cu: the tensor-core F-stage (8192-point windows, 2-bit real, FP16 / FP8 output).
 int fstage_tc_supported(const Job &job, int chan_type);
+// Whether fstage_tc_kernel can address a block of T FFTs: it steps from channel to channel (four channel tiles on) with 32
+// bits of bytes, fstage_tc_cross_kernel with 64.
+inline bool fstage_tc_addresses(int nant, int T, int chan_type) {
+  return (unsigned long long)T * 2 * nant * CW * 4 * chan_elem_bytes(chan_type) <= 0xffffffffull;
+}
 cudaError_t make_fstage_tc_tables(void **out);  // its constant operands (cudaMalloc'd; caller frees)
 // probe non-null: the decode probe (every decoded sample also written to probe [nant][2][nfft][F]).
 cudaError_t launch_fstage_tc(const Job &job, const void *tables, int t0, int nt, int T, void *chan, int chan_type,

@@ -50,6 +50,17 @@ def test_fp16_and_fp8_engines(precision):
     assert _kernel(4, 8192, 3000, precision) == ("cuda_core", "fstage_h_kernel")
 
 
+def test_block_beyond_32_bit_channel_steps():
+    """Spectra of 2^38 bytes: four channel tiles of a block are 2^32 bytes, more than fstage_tc_kernel steps over.  The handle
+    is only made here; it takes the kernel that addresses it."""
+    import torch
+    torch.cuda.empty_cache()
+    if torch.cuda.mem_get_info()[0] < 2 ** 38 + (3 << 30):
+        pytest.skip("needs 278 GB of free device memory")
+    assert _kernel(64, 4096, 131072, "fp16", fft_block=131071)[1] == "fstage_tc_kernel"
+    assert _kernel(64, 4096, 131072, "fp16", fft_block=131072)[1] == "fstage_tc_cross_kernel"
+
+
 @pytest.mark.parametrize("precision", ["fp16", "fp8"])
 @pytest.mark.parametrize("nchan", [1024, 4096])
 def test_choice_does_not_hang_on_the_antenna_count(nchan, precision):
