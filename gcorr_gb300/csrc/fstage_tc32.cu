@@ -372,7 +372,8 @@ __global__ void __launch_bounds__(Plan<L>::NT, 1) fstage_tc32_kernel(Params p) {
         for (int kk = 0; kk < 4; kk++) {
           const int k = 4 * h + kk;
           P2 u[NPR];
-          __syncwarp();  // tensor memory is read by whole warps; put() branches by lane in a group that the block's end cuts
+          // tensor memory is read by whole warps; put() branches by lane in a group whose last windows the block's end cuts off
+          if constexpr (NW > 1) __syncwarp();
 #pragma unroll
           for (int pr = 0; pr < NPR; pr++) {
             ld2(tr + 16 * pr + 2 * k, u[pr].re);
