@@ -31,12 +31,9 @@
 // What bounds it (16 antennas, 2048 FFTs, ncu): 20 warp instructions per 32 samples at 56 % issue active, FMA pipe
 // 40 %, tensor pipe 45 %, shared-memory data path 40 % + 28 % for MMA operands, DRAM 28 %; a window holds its
 // tensor-memory slot for about 9,300 clocks (MMAs, 3,400 for the twiddle, 2,500 for the output), and two slots give
-// one window per 4,850.  F-stage of the 16-antenna, nchan-4096 workload, FP16, 31250 FFTs: 7.4 ms; 15.5 ms for the
-// form before it (one 512-thread CTA that went through the phases of a window together, the intermediate in shared
-// memory written by 2-byte stores); 20.0 ms for the CUDA-core FFT.  Intermediate forms: two 256-thread groups, each
-// one window through all phases, 10.2 ms; warp roles with a block-diagonal M = 128 step 1, 8.1 ms; 16 warps that
-// twiddle two windows and then write two out, 8.6 ms; half windows in 128-column slots, 9.3 ms (a 64-column MMA
-// takes as long as a 128-column one).
+// one window per 4,850.  F-stage of the 16-antenna, nchan-4096 workload, FP16, 31250 FFTs: 7.4 ms; 15.5 ms for
+// fstage_tc_cross_kernel (one 512-thread CTA that goes through the phases of a window together, the intermediate in shared
+// memory written by 2-byte stores); 20.0 ms for the register FFT.
 //
 // Every mbarrier wait is bounded; on expiry the kernel sets an error flag (read by gxc_sync as GXC_ERR_TIMEOUT), lets
 // issued MMAs drain, frees tensor memory and returns.

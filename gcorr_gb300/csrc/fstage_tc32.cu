@@ -32,13 +32,9 @@
 // slots are in flight, connected by mbarriers.
 //
 // What bounds it (16 antennas, 8192 points, FP32, 2048 FFTs, ncu): 40.5 instructions per sample and polarisation (53 for the
-// packed register FFT) at 73 % issue active, FMA pipe 58 % (twiddles and butterflies), tensor pipe 29 %, DRAM 35 %.  While a
-// slot had 48 MMAs (M = 64, 64 clocks each) a team waited 3,600 clocks per group for them; now they are 32.
-// F-stage of the 16-antenna, nchan-4096 workload (62500 FFTs), FP32: 24.3 ms; 40.8 ms for the register FFT (fstage_pair_kernel); 6 antennas, nchan
-// 1024, 15625 FFTs: 0.57 against 0.98 ms.  On the way: eight transform warps on one group at a time, A1 rebuilt for every
-// window, 29.9 ms; the slope check with two decode teams 33.1 ms (the B1 of a slot then waits for its own MMAs); teams on
-// alternate groups 32.4; the MMA descriptors as two words 29.0; the one-word-past loads issued as one instead of a chain
-// 27.1; 16 transform warps, radix 8 x 16 instead of 16 x 8 (half the registers) 26.2.
+// packed register FFT) at 73 % issue active, FMA pipe 58 % (twiddles and butterflies), tensor pipe 29 %, DRAM 35 %.
+// F-stage of the 16-antenna, nchan-4096 workload (62500 FFTs), FP32: 24.4 ms; 40.8 ms for the register FFT
+// (fstage_pair_kernel); 6 antennas, nchan 1024, 15625 FFTs: 0.58 against 0.98 ms.
 //
 // From 16384 points on (N1 = 128) a group is one window; D1 is 128 rows of one polarisation, M = 128 MMAs over two K blocks,
 // and A1 (128 KB) is single, shared by both polarisations and by all windows of the same slope.  At 16384 points team and
@@ -734,8 +730,8 @@ static cudaError_t launch_t(const Params &p, cudaStream_t s) {
 }  // namespace f32tc
 
 // 2048 and 4096 points of 2-bit real data, and 8192 to 32768 points with FP32 output (FP16 and FP8 spectra of 8192
-// points have fstage_tc_kernel; those of 16384 and 32768 points keep fstage_h_kernel, whose FP16 roundings between passes
-// are part of what they are).  At 1024 points, whose rows
+// points have fstage_tc_kernel; those of 16384 and 32768 points keep fstage_h_kernel: without its FP16 roundings between
+// passes their results would move).  At 1024 points, whose rows
 // hold 8 channels, it measured no faster than the register FFT: 61.4 against 63.5 us for 12 groups per SM.  The
 // rotator's phase must be linear over the samples n2 of a row and over the rows: always so in exact mode, in fxkernel
 // mode when the table split is at N2 samples (8192 and 32768 points).  The output addresses use a 32-bit channel step.
