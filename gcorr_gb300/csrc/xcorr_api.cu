@@ -154,7 +154,7 @@ extern "C" gxc_status gxc_xcorr(const float *ants, int nant, int nfft, int nchan
   const float2 *src = ants_dev ? (const float2 *)ants : dants;
   float2 *dst = out_dev ? (float2 *)accum : dout;
   // Where TMA can read the caller's layout, one launch does it all: no re-laid copy (282 of 1000 us at 16 antennas x 1024
-  // channels x 2048 FFTs), no accumulators, and nothing to allocate and free (about 510 us).  190 us instead of 1000.
+  // channels x 2048 FFTs), no accumulators, and nothing to allocate and free (about 510 us).  180 us instead of 1000.
   const bool direct = nvis && engine == GXC_XENGINE_TENSOR && (ants_local || !ants_dev) &&
                       xstage_direct_fits(src, nant, nfft, nchan, fftwidth, ct);
   if (!direct) {

@@ -535,8 +535,8 @@ __global__ void __launch_bounds__(NTHREADS_TC, 1) xstage_tc_kernel(Params p, con
 // Two MMAs per K step, not three: the Gram matrix G = hi.hi^T + lo.hi^T + hi.lo^T is symmetric and its last two terms
 // are each other's transposes, so the stage holds 2 lo, the MMAs accumulate D = hi.hi^T + (2 lo).hi^T, and
 // G = (D + D^T) / 2 is formed once per block.  Fewer truncated additions in TMEM and the mean of two of them: the error
-// against 64 bits falls from 8.9e-7 to 6.5e-7 (6 antennas), 2.8e-6 to 1.9e-6 (TF32 form, 16 antennas).  Time: 10.8 -> 10.7
-// ms (16 antennas, 62500 FFTs, 0.90 of the copy bandwidth), 0.320 -> 0.315 ms (6 antennas, 128 of the 152 SMs); what is
+// against 64 bits falls from 8.9e-7 to 6.5e-7 (6 antennas), 2.8e-6 to 1.9e-6 (TF32 form, 16 antennas).  Time: 10.8 -> 10.5
+// ms (16 antennas, 62500 FFTs, 0.91 of the copy bandwidth), 0.320 -> 0.311 ms (6 antennas, 128 of the 152 SMs); what is
 // left there is the producers' chain of wait, read, split and store.
 constexpr int NEPI_WARPS = 4;
 constexpr int NTHREADS_SPLIT = NPROD + 32 + NEPI_WARPS * 32 + 32;  // + TMA warp (the last)
@@ -554,7 +554,7 @@ constexpr int TMA_WARP_SPLIT = NPROD_WARPS + 1 + NEPI_WARPS;
 // them, [stream][FFT][channel]: 3 is the TF32 split; 2 rounds to FP16 (the precision FP16 of data that arrives in FP32)
 // and needs no lo tile.  Their TMA boxes run through the FFTs of a stream before the next stream, since streams lie
 // megabytes apart: with the stream inside, every row of 16 to 128 bytes was in another page, and 16 antennas x 1024
-// channels x 2048 FFTs took 473 us a call, now 183.  The raw tile then is [stream][FFT][channels]; a warp's lanes take
+// channels x 2048 FFTs took 473 us a call, now 180.  The raw tile then is [stream][FFT][channels]; a warp's lanes take
 // different K chunks o of a stream, and each lane reads its FFTs in an order turned by a function of o, so that eight
 // lanes meet eight banks of 16 bytes.  The order within a K chunk is the same for every row, which a Gram sum allows.
 template <int R, int FORM>

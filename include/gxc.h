@@ -63,7 +63,7 @@ enum { GXC_XENGINE_AUTO = 0, GXC_XENGINE_CUDA_CORE = 1, GXC_XENGINE_TENSOR = 2 }
  * FFT.  CUDA_CORE: the FP32 register FFT of every shape.  AUTO: TENSOR where it
  * runs (16 antennas, nchan 4096, 62500 FFTs, FP16: 14.8 ms per sub-integration, 40 for
  * CUDA_CORE), else MIXED where it is faster, else CUDA_CORE.  Handles without
- * autocorrelations run TENSOR in an earlier form of twice the time (29 ms here), and
+ * autocorrelations run TENSOR in an earlier form of twice the time (31 ms here), and
  * FP8 ones CUDA_CORE for MIXED: their products, mostly noise, keep the roundings of the
  * spectra that they have always had (2-norm of the change otherwise 1e-4 to 1e-3).  MIXED, an answer of
  * gxc_fft_engine and not a choice: the FFT in FP32 accuracy with its first step on
